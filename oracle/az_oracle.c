@@ -162,7 +162,8 @@ static float sample_perlin(const az_texture *t, v3 p) {      /* :156-195 */
         for (int32_t y = 0; y < 2; y++)
             for (int32_t x = 0; x < 2; x++) {
                 uint32_t h = perlin_hash(t->Perm, I + x, J + y, K + z);
-                v3 e = mk(g_gradients[3 * h], g_gradients[3 * h + 1], g_gradients[3 * h + 2]);
+                /* closest-hit queries need no gradients: ids and distances do not depend on bump normals */
+                v3 e = g_gradients ? mk(g_gradients[3 * h], g_gradients[3 * h + 1], g_gradients[3 * h + 2]) : mk(0, 0, 0);
                 v3 v = mk(p.x - (float)(I + x), p.y - (float)(J + y), p.z - (float)(K + z));
                 r += dot(e, v) * perlin_weight(v.x) * perlin_weight(v.y) * perlin_weight(v.z);
             }
