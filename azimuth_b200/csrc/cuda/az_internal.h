@@ -49,10 +49,9 @@ struct GpuScene {
     bool from_soup = false;      // meshes came from az_gpu_scene_create_from_meshes
     size_t device_bytes = 0;
     WaveBuffers waves;           // reused across render calls on this scene
-    uint32_t variant = 7;        // traversal launch configuration, 0-based (128 threads, 8 blocks/SM,
-                                 // persistent fetching; az_gpu_autotune picks per scene)
-    uint32_t shadow_variant = 0xFFFFFFFFu;   // the shadow queries' own configuration (az_gpu_autotune;
-                                             // 0xFFFFFFFF: `variant`)
+    uint32_t variant = 7;        // traversal launch configuration, 0-based (ChooseDefaultVariants; az_gpu_autotune
+                                 // picks per scene)
+    uint32_t shadow_variant = 0xFFFFFFFFu;   // the shadow queries' own configuration (0xFFFFFFFF: `variant`)
     uint32_t order = 0;          // queue ordering (kOrderShadow | kOrderExtend); az_gpu_autotune picks
     az_pixel *host_film_dev = nullptr;   // device film of az_gpu_render_host
     size_t host_film_bytes = 0;
@@ -115,6 +114,8 @@ int CollapseToWide(const azd::BVHNode *d_nodes, const uint2 *d_range, uint32_t b
                    azd::WideNode *d_wide, uint32_t wide_cap, uint32_t *wide_count, uint32_t *d_out_perm,
                    cudaStream_t st, uint32_t *root_out, uint32_t *depth_out);
 
+// The launch configurations a scene starts with, by the size of its hierarchy.
+void ChooseDefaultVariants(GpuScene &G);
 int SetupCamera(const az_camera *c, az_scissor sc, int32_t filter, uint32_t cull, const az_epsilon_values *eps,
                 uint64_t seed, CameraParams &cam);
 // Path guide (az_guide.cu): network state and the hooks of a guided render.

@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "az_internal.h"
+#include "az_phase.cuh"
 #include "az_render.h"
 #include "az_shade.cuh"
 #include "az_wave.cuh"
@@ -99,49 +100,6 @@ __global__ void k_camera_tiles(const Tile *tiles, uint32_t ntiles, uint32_t *nex
     }
 }
 
-// Persistent traversal kernels.  Each warp reserves rays of the level's queue
-// in batches; a lane whose query has finished takes the next reserved ray at
-// its next step, so no lane idles until its warp's slowest ray is done.
-constexpr uint32_t kFetchBatch = 64;
-constexpr uint32_t kLaneIdle = 0xFFFFFFFFu, kLaneDone = 0xFFFFFFFEu;
-
-struct WarpFetch {
-    uint32_t next = 0, end = 0;
-    bool exhausted = false;
-
-    // Hands the idle lanes of the warp new indices below n (kLaneDone when the
-    // queue is exhausted).  Called by all 32 lanes.
-    __device__ __forceinline__ bool refill(uint32_t *counter, uint32_t n, uint32_t &idx) {
-        const uint32_t lane = threadIdx.x & 31u;
-        const uint32_t idle = __ballot_sync(0xFFFFFFFFu, idx == kLaneIdle);
-        if (!idle) return false;
-        if (next >= end && !exhausted) {
-            uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(counter, kFetchBatch);
-            base = __shfl_sync(0xFFFFFFFFu, base, 0);
-            if (base >= n) {
-                exhausted = true;
-            } else {
-                next = base;
-                end = min(base + kFetchBatch, n);
-            }
-        }
-        const uint32_t avail = end - next;
-        bool got = false;
-        if (idx == kLaneIdle) {
-            const uint32_t rank = __popc(idle & ((1u << lane) - 1u));
-            if (rank < avail) {
-                idx = next + rank;
-                got = true;
-            } else if (exhausted) {
-                idx = kLaneDone;
-            }
-        }
-        next += min(avail, (uint32_t)__popc(idle));
-        return got;
-    }
-};
-
 // Sort keys that group a level's queue by where its rays start: a 15-bit
 // Morton code of the origin's cell in a 32^3 grid over the scene bounds, for
 // extension rays the top 13 bits of it and the direction octant.  Entries past
@@ -177,119 +135,194 @@ __global__ void k_order_keys(DevScene S, WaveQueues Q, uint32_t level, int shado
     }
 }
 
-// How a traversal kernel maps queries to threads:
-//   MODE_LOOP     one query per thread at a time in a grid-stride loop, each
-//                 thread running its query to the end in one loop
-//   MODE_LOCKSTEP the same assignment, but the warp advances its 32 queries
-//                 one traversal step at a time and reconverges after every
-//                 step
-//   MODE_FETCH    persistent warps: a lane takes the next query of the queue
-//                 as soon as its own ends (batches of kFetchBatch per warp)
-//   MODE_FETCHP   the same, with traversal steps that pop the stack first
-//                 and visit the popped group in the same step (Tracer
-//                 POP_FIRST), so lanes coming back from a pop join the
-//                 warp's node visits instead of idling through them
-//   MODE_STAGED   MODE_FETCHP with the node fetches of each step staged
-//                 through shared memory by the whole warp (stage_nodes)
-enum : int { MODE_LOOP = 0, MODE_LOCKSTEP = 1, MODE_FETCH = 2, MODE_FETCHP = 3, MODE_STAGED = 4 };
+// When a warp of the traversal kernels does what (az_phase.cuh): finished lanes
+// wait until `refill` of them can write their results and take new queries
+// together (LaunchParams); primitives are tested once kPrimLanes lanes hold
+// some, or at least as many as could visit a node, and for as long as
+// kPrimStay do.  Measured on full frames of the dense mesh, the interior and the
+// moving spheres (one B200): kPrimLanes 10: 211 / 296 / 169 ms, 12: 210 / 292 /
+// 170, 16: 208 / 287 / 172.
+constexpr uint32_t kPrimLanes = 16, kPrimStay = 8;
+constexpr uint32_t kFetchBatch = 64;   // queries a warp takes from the queue at once
+constexpr uint32_t kNoQuery = 0xFFFFFFFFu;
+constexpr int kTraceBlock = 128;       // threads a block of the traversal kernels
 
-// WT: triangles by the watertight test (AZ_FLAG_WATERTIGHT) instead of azimuth's.
-// MULTI: a tile wave of several scenes (persistent modes only): each query is
-// traced in the scene its entry names (WaveQueues.scenes).
-// SPH: the top-level sphere test inline (Tracer SPH).
-template <int BLOCK, int MINB, int MODE, bool WT = false, bool MULTI = false, bool SPH = false>
-__global__ void __launch_bounds__(BLOCK, MINB) k_extend(DevScene S, CameraParams cam, WaveQueues Q, uint32_t level) {
-    const int buf = level & 1;
-    const uint32_t n = min(Q.counts[level], Q.cap_q);
-    uint32_t *cnt = cam.count_traversal ? Q.counts + AZ_COUNT_NODES : nullptr;
-    uint32_t *err = Q.counts + AZ_COUNT_ERROR;
-    if (MODE == MODE_LOCKSTEP) {
-        Tracer<Q_CLOSEST, false, WT, SPH> T;
-        uint2 stack[AZD_WSTACK];
-        // warp-uniform loop bound: every lane of a warp sees the same base
-        for (uint32_t base = blockIdx.x * BLOCK + (threadIdx.x & ~31u); base < n; base += gridDim.x * BLOCK) {
-            const uint32_t k = base + (threadIdx.x & 31u);
-            bool live = k < n;
-            const uint32_t i = live && Q.eorder ? Q.eorder[k] : k;
-            if (live) {
-                const float4 o = Q.o[buf][i], d = Q.d[buf][i];
-                Ray r;
-                r.o = mk(o.x, o.y, o.z);
-                r.d = mk(d.x, d.y, d.z);
-                r.time = o.w;
-                T.init(S, r, cam.cull != 0, cam.eps_isect, FLT_MAX, stack);
-            }
-            while (__any_sync(0xFFFFFFFFu, live)) {
-                if (live && T.step(S, stack, err)) {
-                    const Hit &h = T.best;
-                    Q.hit[i] = make_uint4(__float_as_uint(h.t), __float_as_uint(h.tl), h.prim, h.ent);
-                    T.flush_counts(cnt);
-                    live = false;
+// The loop of a phase-scheduled kernel: called by all 32 lanes of a warp.
+//   load(q)          the world ray of queue entry q
+//   begin(q)         starts its query; false when this kernel leaves it out
+//   end(q)           writes the result of a finished query; false: it goes on
+//   size             the queue's length (in device memory), at most cap
+//   order            the queue's visiting order or null
+template <bool COUNT, typename TRACER, typename LOAD, typename BEGIN, typename END, typename SCENE>
+__device__ __forceinline__ void phase_run(TRACER &T, const uint32_t *size, uint32_t cap, const uint32_t *order,
+                                          uint32_t *fetch, uint32_t refill, bool cull, float eps, LOAD load,
+                                          BEGIN begin, END end, SCENE scene, uint32_t *err,
+                                          uint32_t *counts) {
+    constexpr uint32_t kAll = 0xFFFFFFFFu;
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t qi = kNoQuery;            // this lane's queue entry
+    bool done = false;                 // its query has finished
+    uint32_t next = 0, last = 0;       // the warp's batch of work items; kNoQuery: the queue is exhausted
+    uint32_t nodes_seen = 0, prims_seen = 0;
+    auto ray = [&]() { return load(qi); };
+    for (;;) {
+        if (done) {
+            done = false;
+            if (end(qi)) qi = kNoQuery;
+        }
+        uint32_t idle = __ballot_sync(kAll, qi == kNoQuery);
+        while (idle && last != kNoQuery) {
+            if (next == last) {
+                // batches small enough that the launch's warps share a short queue evenly
+                const uint32_t n = min(*size, cap);
+                const uint32_t batch = min(kFetchBatch, max(32u, n / (gridDim.x * (blockDim.x >> 5) * 2u)));
+                if (lane == 0) next = atomicAdd(fetch, batch);
+                next = __shfl_sync(kAll, next, 0);
+                last = min(next + batch, n);
+                if (next >= n) {
+                    next = last = kNoQuery;
+                    break;
                 }
             }
+            const uint32_t k = next + __popc(idle & ((1u << lane) - 1u));
+            if ((idle >> lane) & 1u && k < last) {
+                const uint32_t q = order ? order[k] : k;
+                if (begin(q)) qi = q;
+            }
+            next = min(last, next + (uint32_t)__popc(idle));
+            idle = __ballot_sync(kAll, qi == kNoQuery);
         }
-        return;
+        // rounds until enough lanes wait (all of the idle ones are idle for good)
+        const uint32_t spare = __popc(idle);
+        if (spare == 32u) break;
+        for (uint32_t rounds = 0;; rounds++) {
+            if (rounds > AZD_MAX_STEPS) {
+                // far more than a valid hierarchy needs: give up on these queries and on the rest
+                if (qi != kNoQuery && !done) {
+                    atomicOr(err, 1u);
+                    T.abandon();
+                }
+                next = last = kNoQuery;
+            }
+            bool live = qi != kNoQuery && !done;
+            if (live && T.refill(scene(), ray, eps)) {
+                done = true;
+                live = false;
+            }
+            const uint32_t nodes = __ballot_sync(kAll, live && T.wants_node());
+            uint32_t prims = __ballot_sync(kAll, live && T.has_prims());
+            const uint32_t busy = __popc(nodes | prims);
+            if (!busy || 32u - busy - spare >= refill) break;
+            const uint32_t np = __popc(prims);
+            if (np >= kPrimLanes || (np && np >= __popc(nodes))) {
+                do {
+                    if (COUNT) prims_seen += __popc(prims);
+                    if (live && T.has_prims() && T.prim(scene(), ray, cull, eps, err)) {
+                        done = true;
+                        live = false;
+                    }
+                    prims = __ballot_sync(kAll, live && T.has_prims());
+                } while (__popc(prims) >= kPrimStay);
+            } else {
+                if (COUNT) nodes_seen += __popc(nodes);
+                if (live && T.wants_node()) T.node(scene(), err);
+            }
+        }
     }
-    if (MODE == MODE_LOOP) {
-        // one query per thread at a time, grid-stride over the queue
-        for (uint32_t k = blockIdx.x * BLOCK + threadIdx.x; k < n; k += gridDim.x * BLOCK) {
+    if (COUNT && lane == 0) {
+        atomicAdd(counts + 0, nodes_seen);
+        atomicAdd(counts + 1, prims_seen);
+    }
+}
+
+// Closest hits of the level's queue.
+// WT: triangles by the watertight test (AZ_FLAG_WATERTIGHT) instead of azimuth's.
+// MULTI: a tile wave of several scenes: each query is traced in the scene its
+// entry names (WaveQueues.scenes).
+// SPH: the scene has spheres at the top level (DevScene.top_spheres).
+// COUNT: visit counters (AZ_FLAG_COUNT_TRAVERSAL).
+// Bound by the issue of divergent instructions (profiles/): 128 threads of at
+// most 64 registers, 32 warps a multiprocessor, no spills.
+//
+// MINB == 0: one query per thread in a grid-stride loop, for scenes whose whole
+// hierarchy is a few nodes: all lanes then take nearly the same steps, and the
+// votes and the shared stack cost more than they give (Cornell box, 1 M samples:
+// closest hits 0.48 ms a frame against 0.65).
+template <int MINB, bool WT, bool MULTI, bool SPH, bool COUNT>
+__global__ void __launch_bounds__(kTraceBlock, MINB ? MINB : 8)
+    k_extend(DevScene S, CameraParams cam, WaveQueues Q, uint32_t level) {
+    if constexpr (MINB == 0) {
+        const uint32_t n = min(Q.counts[level], Q.cap_q);
+        for (uint32_t k = blockIdx.x * kTraceBlock + threadIdx.x; k < n; k += gridDim.x * kTraceBlock) {
             const uint32_t i = Q.eorder ? Q.eorder[k] : k;
-            const float4 o = Q.o[buf][i], d = Q.d[buf][i];
+            const float4 o = Q.o[level & 1][i], d = Q.d[level & 1][i];
             Ray r;
             r.o = mk(o.x, o.y, o.z);
             r.d = mk(d.x, d.y, d.z);
             r.time = o.w;
             Hit h;
-            trace<Q_CLOSEST, WT>(S, r, cam.cull != 0, cam.eps_isect, FLT_MAX, h, cnt, err);
+            trace<Q_CLOSEST, WT>(S, r, cam.cull != 0, cam.eps_isect, FLT_MAX, h,
+                                 COUNT ? Q.counts + AZ_COUNT_NODES : nullptr, Q.counts + AZ_COUNT_ERROR);
             Q.hit[i] = make_uint4(__float_as_uint(h.t), __float_as_uint(h.tl), h.prim, h.ent);
         }
         return;
     }
-    uint32_t *fetch = Q.counts + AZ_COUNT_FETCH + level;
-    constexpr bool STAGED = MODE == MODE_STAGED;
-    static_assert(!(STAGED && MULTI), "staged fetching serves one scene");
-    __shared__ uint4 s_stage[STAGED ? BLOCK / 32 * 160 : 1];
-    Tracer<Q_CLOSEST, MODE == MODE_FETCHP || STAGED, WT, SPH> T;
-    uint2 stack[AZD_WSTACK];
-    WarpFetch wf;
-    uint32_t idx = kLaneIdle, qi = 0;   // work item and its queue entry
-    uint32_t si = 0;                    // MULTI: the entry's scene
-    while (true) {
-        if (wf.refill(fetch, n, idx)) {
-            qi = Q.eorder ? Q.eorder[idx] : idx;
-            const float4 o = Q.o[buf][qi], d = Q.d[buf][qi];
-            Ray r;
-            r.o = mk(o.x, o.y, o.z);
-            r.d = mk(d.x, d.y, d.z);
-            r.time = o.w;
-            if (MULTI) si = (__float_as_uint(d.w) & PF_SCENE) >> PF_SCENE_SHIFT;
-            T.init(MULTI ? Q.scenes[si] : S, r, cam.cull != 0, cam.eps_isect, FLT_MAX, stack);
-        }
-        if (__all_sync(0xFFFFFFFFu, idx == kLaneDone)) break;
-        bool fin;
-        if (STAGED) {
-            const bool live = idx < n;
-            uint32_t node = T.kNoNode;
-            fin = live && T.begin(S, stack, err, node);
-            uint4 w[5];
-            stage_nodes(S.wnodes, node, s_stage + (threadIdx.x >> 5) * 160u, w);
-            fin = live && (fin || T.finish(S, stack, err, node, w));
-        } else {
-            fin = idx < n && T.step(MULTI ? Q.scenes[si] : S, stack, err);
-        }
-        if (fin) {
-            const Hit &h = T.best;
-            Q.hit[qi] = make_uint4(__float_as_uint(h.t), __float_as_uint(h.tl), h.prim, h.ent);
-            T.flush_counts(cnt);
-            idx = kLaneIdle;
-        }
+    __shared__ PhaseShared<kTraceBlock> shared;
+    uint2 deep[AZD_WSTACK - kSharedStack];
+    PhaseTracer<Q_CLOSEST, WT, SPH, kTraceBlock> T(shared, deep);
+    const int buf = level & 1;
+    uint32_t si = 0;   // MULTI: the entry's scene
+    auto load = [&](uint32_t q) {
+        const float4 o = Q.o[buf][q], d = Q.d[buf][q];
+        Ray r;
+        r.o = mk(o.x, o.y, o.z);
+        r.d = mk(d.x, d.y, d.z);
+        r.time = o.w;
+        if (MULTI) si = (__float_as_uint(d.w) & PF_SCENE) >> PF_SCENE_SHIFT;
+        return r;
+    };
+    auto scene = [&]() -> const DevScene & { return MULTI ? Q.scenes[si] : S; };
+    auto begin = [&](uint32_t q) {
+        const Ray r = load(q);
+        T.init(scene(), r, FLT_MAX, 0xFFFFFFFFu);
+        return true;
+    };
+    auto end = [&](uint32_t q) {
+        if (T.in_blas) T.take_group_hit(scene(), load(q), cam.eps_isect);
+        Q.hit[q] = T.hit();
+        return true;
+    };
+    phase_run<COUNT>(T, Q.counts + level, Q.cap_q, Q.eorder, Q.counts + AZ_COUNT_FETCH + level, cam.refill,
+                     cam.cull != 0, cam.eps_isect, load, begin, end, scene, Q.counts + AZ_COUNT_ERROR,
+                     Q.counts + AZ_COUNT_NODES);
+}
+
+// Entity lights: a light sample is occluded unless the nearest hit is the
+// light's entity, so the light's own nearest hit is found first and the
+// visibility query looks for anything else before it.  This kernel replaces the
+// limit of the level's SHADOW_ENTITY queries by that distance (FLT_MAX: the ray
+// misses the light).  Inside k_shadow the light's test ran with the few lanes
+// that took a new query at a time and its call spilled the traversal's
+// registers: C1's visibility queries take 66 ms a frame after this pass (of
+// 2-3 ms, bound by the 36 bytes it reads per query) against 80 ms.
+template <bool MULTI>
+__global__ void __launch_bounds__(256) k_light_limits(DevScene S0, WaveQueues Q, uint32_t level) {
+    const uint32_t n = min(Q.counts[AZ_COUNT_SHADOW + level], Q.cap_s);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t meta = Q.smeta[i];
+        if (shadow_kind(meta) != SHADOW_ENTITY) continue;
+        const DevScene &S = MULTI ? Q.scenes[shadow_scene(meta)] : S0;
+        const float4 o = Q.so[i], d = Q.sd[i];
+        Ray r;
+        r.o = mk(o.x, o.y, o.z);
+        r.d = mk(d.x, d.y, d.z);
+        r.time = o.w;
+        float t = FLT_MAX;
+        light_entity_hit(S.ents, S.light_tris, S.lights[shadow_light(meta)], r, t);
+        Q.sd[i].w = t;
     }
 }
 
-// Visibility of the queued light samples; unoccluded ones are added to their
-// sample.  Entity lights: occluded unless the nearest hit is the light's
-// entity, so the light's own nearest hit is found exactly first and the query
-// looks for anything else before it.
 // Visibility of the SHADOW_ENTITY_FULL queries of the shadow queue (entity
 // lights too large for the two-phase test): one full nearest-hit query each,
 // visible when the nearest hit is the light's entity (src/azimuth_main.cpp:694-712).
@@ -315,122 +348,65 @@ __global__ void __launch_bounds__(128) k_shadow_full(DevScene S0, CameraParams c
     }
 }
 
-template <int BLOCK, int MINB, int MODE, bool WT = false, bool MULTI = false, bool SPH = false>
-__global__ void __launch_bounds__(BLOCK, MINB) k_shadow(DevScene S, CameraParams cam, WaveQueues Q, uint32_t level) {
-    const uint32_t n = min(Q.counts[AZ_COUNT_SHADOW + level], Q.cap_s);
-    uint32_t *cnt = cam.count_traversal ? Q.counts + AZ_COUNT_SNODES : nullptr;
-    uint32_t *err = Q.counts + AZ_COUNT_ERROR;
-    if (MODE == MODE_LOCKSTEP) {
-        Tracer<Q_ANY, false, WT, SPH> T;
-        uint2 stack[AZD_WSTACK];
-        for (uint32_t base = blockIdx.x * BLOCK + (threadIdx.x & ~31u); base < n; base += gridDim.x * BLOCK) {
-            const uint32_t k = base + (threadIdx.x & 31u);
-            bool live = k < n;
-            const uint32_t i = live && Q.sorder ? Q.sorder[k] : k;
-            float4 c = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (live) {
-                const float4 o = Q.so[i], d = Q.sd[i];
-                c = Q.sc[i];
-                const uint32_t meta = Q.smeta[i];
-                const uint32_t kind = shadow_kind(meta), li = shadow_light(meta);
-                Ray r;
-                r.o = mk(o.x, o.y, o.z);
-                r.d = mk(d.x, d.y, d.z);
-                r.time = o.w;
-                if (kind == SHADOW_ENTITY_FULL) {
-                    live = false;   // k_shadow_full
-                } else if (kind == SHADOW_ENTITY) {
-                    const LightHit lh = light_entity_hit_call(S.ents, S.light_tris, S.lights + li, r);
-                    T.init(S, r, false, 0.0f, lh.hit ? lh.t : FLT_MAX, stack, S.lights[li].ent_index);
-                } else {
-                    T.init(S, r, false, 0.0f, kind == SHADOW_ANY ? FLT_MAX : d.w, stack);
-                }
-            }
-            while (__any_sync(0xFFFFFFFFu, live)) {
-                if (live && T.step(S, stack, err)) {
-                    if (!T.hit_any) add_accum(Q.accum, __float_as_uint(c.w), mk(c.x, c.y, c.z));
-                    T.flush_counts(cnt);
-                    live = false;
-                }
-            }
-        }
-        return;
-    }
-    if (MODE == MODE_LOOP) {
-        for (uint32_t k = blockIdx.x * BLOCK + threadIdx.x; k < n; k += gridDim.x * BLOCK) {
+// Visibility of the queued light samples; unoccluded ones are added to their
+// sample.  Template arguments as k_extend.
+template <int MINB, bool WT, bool MULTI, bool SPH, bool COUNT>
+__global__ void __launch_bounds__(kTraceBlock, MINB ? MINB : 8)
+    k_shadow(DevScene S, CameraParams cam, WaveQueues Q, uint32_t level) {
+    if constexpr (MINB == 0) {
+        const uint32_t n = min(Q.counts[AZ_COUNT_SHADOW + level], Q.cap_s);
+        for (uint32_t k = blockIdx.x * kTraceBlock + threadIdx.x; k < n; k += gridDim.x * kTraceBlock) {
             const uint32_t i = Q.sorder ? Q.sorder[k] : k;
             const float4 o = Q.so[i], d = Q.sd[i], c = Q.sc[i];
             const uint32_t meta = Q.smeta[i];
-            const uint32_t kind = shadow_kind(meta), li = shadow_light(meta);
+            const uint32_t kind = shadow_kind(meta);
+            if (kind == SHADOW_ENTITY_FULL) continue;   // k_shadow_full
             Ray r;
             r.o = mk(o.x, o.y, o.z);
             r.d = mk(d.x, d.y, d.z);
             r.time = o.w;
             Hit h;
-            bool visible;
-            if (kind == SHADOW_ENTITY_FULL) {
-                continue;   // k_shadow_full
-            } else if (kind == SHADOW_ENTITY) {
-                const LightHit lh = light_entity_hit_call(S.ents, S.light_tris, S.lights + li, r);
-                visible = !trace<Q_ANY, WT>(S, r, false, 0.0f, lh.hit ? lh.t : FLT_MAX, h, cnt, err,
-                                            S.lights[li].ent_index);
-            } else {
-                visible = !trace<Q_ANY, WT>(S, r, false, 0.0f, kind == SHADOW_ANY ? FLT_MAX : d.w, h, cnt, err);
-            }
-            if (visible) add_accum(Q.accum, __float_as_uint(c.w), mk(c.x, c.y, c.z));
+            if (!trace<Q_ANY, WT>(S, r, false, 0.0f, kind == SHADOW_ANY ? FLT_MAX : d.w, h,
+                                  COUNT ? Q.counts + AZ_COUNT_SNODES : nullptr, Q.counts + AZ_COUNT_ERROR,
+                                  kind == SHADOW_ENTITY ? S.lights[shadow_light(meta)].ent_index : 0xFFFFFFFFu))
+                add_accum(Q.accum, __float_as_uint(c.w), mk(c.x, c.y, c.z));
         }
         return;
     }
-    uint32_t *fetch = Q.counts + AZ_COUNT_FETCH + AZ_MAX_LEVELS + level;
-    constexpr bool STAGED = MODE == MODE_STAGED;
-    static_assert(!(STAGED && MULTI), "staged fetching serves one scene");
-    __shared__ uint4 s_stage[STAGED ? BLOCK / 32 * 160 : 1];
-    Tracer<Q_ANY, MODE == MODE_FETCHP || STAGED, WT, SPH> T;
-    uint2 stack[AZD_WSTACK];
-    WarpFetch wf;
-    uint32_t idx = kLaneIdle;
+    __shared__ PhaseShared<kTraceBlock> shared;
+    uint2 deep[AZD_WSTACK - kSharedStack];
+    PhaseTracer<Q_ANY, WT, SPH, kTraceBlock> T(shared, deep);
     uint32_t si = 0;   // MULTI: the entry's scene
-    float4 c = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    while (true) {
-        if (wf.refill(fetch, n, idx)) {
-            const uint32_t qi = Q.sorder ? Q.sorder[idx] : idx;
-            const float4 o = Q.so[qi], d = Q.sd[qi];
-            c = Q.sc[qi];
-            const uint32_t meta = Q.smeta[qi];
-            const uint32_t kind = shadow_kind(meta), li = shadow_light(meta);
-            if (MULTI) si = shadow_scene(meta);
-            const DevScene &Sq = MULTI ? Q.scenes[si] : S;
-            Ray r;
-            r.o = mk(o.x, o.y, o.z);
-            r.d = mk(d.x, d.y, d.z);
-            r.time = o.w;
-            if (kind == SHADOW_ENTITY_FULL) {
-                idx = kLaneIdle;   // k_shadow_full
-            } else if (kind == SHADOW_ENTITY) {
-                const LightHit lh = light_entity_hit_call(Sq.ents, Sq.light_tris, Sq.lights + li, r);
-                T.init(Sq, r, false, 0.0f, lh.hit ? lh.t : FLT_MAX, stack, Sq.lights[li].ent_index);
-            } else {
-                T.init(Sq, r, false, 0.0f, kind == SHADOW_ANY ? FLT_MAX : d.w, stack);
-            }
+    auto load = [&](uint32_t q) {
+        const float4 o = Q.so[q], d = Q.sd[q];
+        Ray r;
+        r.o = mk(o.x, o.y, o.z);
+        r.d = mk(d.x, d.y, d.z);
+        r.time = o.w;
+        return r;
+    };
+    auto scene = [&]() -> const DevScene & { return MULTI ? Q.scenes[si] : S; };
+    auto begin = [&](uint32_t q) {
+        const uint32_t meta = Q.smeta[q];
+        const uint32_t kind = shadow_kind(meta);
+        if (MULTI) si = shadow_scene(meta);
+        if (kind == SHADOW_ENTITY_FULL) return false;   // k_shadow_full
+        const Ray r = load(q);
+        T.init(scene(), r, kind == SHADOW_ANY ? FLT_MAX : Q.sd[q].w,   // an entity light's: k_light_limits
+               kind == SHADOW_ENTITY ? scene().lights[shadow_light(meta)].ent_index : 0xFFFFFFFFu);
+        return true;
+    };
+    auto end = [&](uint32_t q) {
+        if (!T.confirm(scene(), load(q), 0.0f)) return false;
+        if (!T.occluded) {
+            const float4 c = Q.sc[q];
+            add_accum(Q.accum, __float_as_uint(c.w), mk(c.x, c.y, c.z));
         }
-        if (__all_sync(0xFFFFFFFFu, idx == kLaneDone)) break;
-        bool fin;
-        if (STAGED) {
-            const bool live = idx < n;
-            uint32_t node = T.kNoNode;
-            fin = live && T.begin(S, stack, err, node);
-            uint4 w[5];
-            stage_nodes(S.wnodes, node, s_stage + (threadIdx.x >> 5) * 160u, w);
-            fin = live && (fin || T.finish(S, stack, err, node, w));
-        } else {
-            fin = idx < n && T.step(MULTI ? Q.scenes[si] : S, stack, err);
-        }
-        if (fin) {
-            if (!T.hit_any) add_accum(Q.accum, __float_as_uint(c.w), mk(c.x, c.y, c.z));
-            T.flush_counts(cnt);
-            idx = kLaneIdle;
-        }
-    }
+        return true;
+    };
+    phase_run<COUNT>(T, Q.counts + AZ_COUNT_SHADOW + level, Q.cap_s, Q.sorder,
+                     Q.counts + AZ_COUNT_FETCH + AZ_MAX_LEVELS + level, cam.shadow_refill, false, 0.0f, load, begin, end,
+                     scene, Q.counts + AZ_COUNT_ERROR, Q.counts + AZ_COUNT_SNODES);
 }
 
 // ComputeSampleWeight (src/azimuth_main.cpp:1209-1254) for every sample of the wave.
@@ -482,91 +458,64 @@ __global__ void k_splat_tiles(WaveQueues Q, uint32_t n, az_pixel *const *films) 
     splat_sample(Q.job_cams[js.x], films[js.x], js.y, Q.accum[i]);
 }
 
-// Launch configurations of the two traversal kernels: threads per block,
-// minimum resident blocks per SM (which caps registers), and whether warps
-// fetch rays persistently (a lane takes a new ray as soon as its query ends)
-// or one query per thread in a grid-stride loop; chosen per scene by
-// az_gpu_autotune.
+// Launch configurations of the two traversal kernels, chosen per scene by
+// az_gpu_autotune: resident blocks per multiprocessor (which caps registers:
+// 7 blocks of 128 threads 72, 8 blocks 64) and the lanes that wait for each
+// other before a warp writes results and takes new queries (32: a warp's
+// queries begin and end together); or one query per thread (0 blocks).
 struct Variant {
-    int block, minb, mode;
+    int minb;
+    uint32_t refill;
 };
-constexpr Variant kVariants[] = {{128, 1, MODE_LOOP},     {128, 6, MODE_LOOP},     {128, 8, MODE_LOOP},
-                                 {256, 1, MODE_LOOP},     {256, 3, MODE_LOOP},     {64, 1, MODE_LOOP},
-                                 {64, 12, MODE_LOOP},     {128, 8, MODE_FETCH},    {128, 6, MODE_FETCH},
-                                 {256, 3, MODE_FETCH},    {128, 8, MODE_LOCKSTEP}, {128, 6, MODE_LOCKSTEP},
-                                 {256, 3, MODE_LOCKSTEP}, {64, 12, MODE_LOCKSTEP}, {128, 7, MODE_FETCH},
-                                 {128, 6, MODE_FETCHP},   {128, 7, MODE_FETCHP},   {128, 8, MODE_FETCHP},
-                                 {128, 6, MODE_STAGED},   {128, 8, MODE_STAGED}};
+constexpr Variant kVariants[] = {{8, 4},  {8, 6},  {8, 10}, {8, 12}, {8, 14}, {8, 16}, {8, 20},
+                                 {8, 8},  {8, 24}, {8, 32}, {0, 32}, {7, 4},  {7, 6},  {7, 8},
+                                 {7, 10}, {7, 12}, {7, 14}, {7, 16}, {7, 24}, {7, 32}};
 constexpr uint32_t kVariantCount = sizeof(kVariants) / sizeof(kVariants[0]);
 static_assert(kVariantCount == AZ_LAUNCH_VARIANTS, "variant table and header disagree");
 
-// Scenes with spheres at the top level get the kernels with the sphere test
-// inline (a one-thread-per-query loop always has it inline).
-template <int B, int M, int P>
+template <int MINB, bool WT, bool MULTI, bool SPH, bool COUNT>
 void LaunchTraversal(bool shadow, int sms, const DevScene &S, const CameraParams &cam, const WaveQueues &Q,
                      uint32_t L, cudaStream_t st) {
-    const int grid = sms * (2048 / B);
-    if (P != MODE_LOOP && S.top_spheres) {
-        if (shadow) k_shadow<B, M, P, false, false, true><<<grid, B, 0, st>>>(S, cam, Q, L);
-        else k_extend<B, M, P, false, false, true><<<grid, B, 0, st>>>(S, cam, Q, L);
-        return;
-    }
-    if (shadow) k_shadow<B, M, P><<<grid, B, 0, st>>>(S, cam, Q, L);
-    else k_extend<B, M, P><<<grid, B, 0, st>>>(S, cam, Q, L);
+    const int grid = sms * (2048 / kTraceBlock);
+    if (shadow) k_shadow<MINB, WT, MULTI, SPH, COUNT><<<grid, kTraceBlock, 0, st>>>(S, cam, Q, L);
+    else k_extend<MINB, WT, MULTI, SPH, COUNT><<<grid, kTraceBlock, 0, st>>>(S, cam, Q, L);
 }
 
+template <int MINB, bool WT, bool MULTI>
+void LaunchTraversal(bool shadow, int sms, const DevScene &S, const CameraParams &cam, const WaveQueues &Q,
+                     uint32_t L, cudaStream_t st) {
+    if (S.top_spheres) {
+        if (cam.count_traversal) LaunchTraversal<MINB, WT, MULTI, true, true>(shadow, sms, S, cam, Q, L, st);
+        else LaunchTraversal<MINB, WT, MULTI, true, false>(shadow, sms, S, cam, Q, L, st);
+    } else {
+        if (cam.count_traversal) LaunchTraversal<MINB, WT, MULTI, false, true>(shadow, sms, S, cam, Q, L, st);
+        else LaunchTraversal<MINB, WT, MULTI, false, false>(shadow, sms, S, cam, Q, L, st);
+    }
+}
+
+// The closest-hit stage of level L, or its visibility stage, in launch
+// configuration v (its blocks per multiprocessor; the lanes are in `cam`).
 void LaunchTraversalVariant(uint32_t v, bool shadow, int sms, const DevScene &S, const CameraParams &cam,
                             const WaveQueues &Q, uint32_t L, cudaStream_t st) {
-    const int fgrid = sms * 16;
-    if (Q.scenes) {
-        // a tile wave of several scenes: one launch configuration, 128 threads, at most 64 registers,
-        // persistent fetching (variant 8), the sphere test inline when any scene has top-level spheres
-        if (cam.watertight) {
-            if (shadow && S.full_light_queries) k_shadow_full<true, true><<<fgrid, 128, 0, st>>>(S, cam, Q, L);
-            if (shadow) k_shadow<128, 8, MODE_FETCH, true, true><<<fgrid, 128, 0, st>>>(S, cam, Q, L);
-            else k_extend<128, 8, MODE_FETCH, true, true><<<fgrid, 128, 0, st>>>(S, cam, Q, L);
-        } else {
-            if (shadow && S.full_light_queries) k_shadow_full<false, true><<<fgrid, 128, 0, st>>>(S, cam, Q, L);
-            if (S.top_spheres) {
-                if (shadow) k_shadow<128, 8, MODE_FETCH, false, true, true><<<fgrid, 128, 0, st>>>(S, cam, Q, L);
-                else k_extend<128, 8, MODE_FETCH, false, true, true><<<fgrid, 128, 0, st>>>(S, cam, Q, L);
-            } else {
-                if (shadow) k_shadow<128, 8, MODE_FETCH, false, true><<<fgrid, 128, 0, st>>>(S, cam, Q, L);
-                else k_extend<128, 8, MODE_FETCH, false, true><<<fgrid, 128, 0, st>>>(S, cam, Q, L);
-            }
-        }
-        return;
+    const int grid = sms * 16;
+    const bool loop = kVariants[v].minb == 0 && !Q.scenes && !cam.watertight;
+    if (shadow && S.entity_lights) {
+        if (Q.scenes) k_light_limits<true><<<sms * 8, 256, 0, st>>>(S, Q, L);
+        else k_light_limits<false><<<sms * 8, 256, 0, st>>>(S, Q, L);
     }
-    if (cam.watertight) {
-        // the watertight test has one launch configuration: 128 threads, pop-first persistent fetching
-        if (shadow && S.full_light_queries) k_shadow_full<true><<<fgrid, 128, 0, st>>>(S, cam, Q, L);
-        if (shadow) k_shadow<128, 6, MODE_FETCHP, true><<<fgrid, 128, 0, st>>>(S, cam, Q, L);
-        else k_extend<128, 6, MODE_FETCHP, true><<<fgrid, 128, 0, st>>>(S, cam, Q, L);
-        return;
+    if (shadow && S.full_light_queries) {
+        if (Q.scenes && cam.watertight) k_shadow_full<true, true><<<grid, 128, 0, st>>>(S, cam, Q, L);
+        else if (Q.scenes) k_shadow_full<false, true><<<grid, 128, 0, st>>>(S, cam, Q, L);
+        else if (cam.watertight) k_shadow_full<true><<<grid, 128, 0, st>>>(S, cam, Q, L);
+        else k_shadow_full<false><<<grid, 128, 0, st>>>(S, cam, Q, L);
     }
-    if (shadow && S.full_light_queries) k_shadow_full<false><<<fgrid, 128, 0, st>>>(S, cam, Q, L);
-    switch (v) {
-        case 0: LaunchTraversal<128, 1, MODE_LOOP>(shadow, sms, S, cam, Q, L, st); break;
-        case 1: LaunchTraversal<128, 6, MODE_LOOP>(shadow, sms, S, cam, Q, L, st); break;
-        case 3: LaunchTraversal<256, 1, MODE_LOOP>(shadow, sms, S, cam, Q, L, st); break;
-        case 4: LaunchTraversal<256, 3, MODE_LOOP>(shadow, sms, S, cam, Q, L, st); break;
-        case 5: LaunchTraversal<64, 1, MODE_LOOP>(shadow, sms, S, cam, Q, L, st); break;
-        case 6: LaunchTraversal<64, 12, MODE_LOOP>(shadow, sms, S, cam, Q, L, st); break;
-        case 7: LaunchTraversal<128, 8, MODE_FETCH>(shadow, sms, S, cam, Q, L, st); break;
-        case 8: LaunchTraversal<128, 6, MODE_FETCH>(shadow, sms, S, cam, Q, L, st); break;
-        case 9: LaunchTraversal<256, 3, MODE_FETCH>(shadow, sms, S, cam, Q, L, st); break;
-        case 10: LaunchTraversal<128, 8, MODE_LOCKSTEP>(shadow, sms, S, cam, Q, L, st); break;
-        case 11: LaunchTraversal<128, 6, MODE_LOCKSTEP>(shadow, sms, S, cam, Q, L, st); break;
-        case 12: LaunchTraversal<256, 3, MODE_LOCKSTEP>(shadow, sms, S, cam, Q, L, st); break;
-        case 13: LaunchTraversal<64, 12, MODE_LOCKSTEP>(shadow, sms, S, cam, Q, L, st); break;
-        case 14: LaunchTraversal<128, 7, MODE_FETCH>(shadow, sms, S, cam, Q, L, st); break;
-        case 15: LaunchTraversal<128, 6, MODE_FETCHP>(shadow, sms, S, cam, Q, L, st); break;
-        case 16: LaunchTraversal<128, 7, MODE_FETCHP>(shadow, sms, S, cam, Q, L, st); break;
-        case 17: LaunchTraversal<128, 8, MODE_FETCHP>(shadow, sms, S, cam, Q, L, st); break;
-        case 18: LaunchTraversal<128, 6, MODE_STAGED>(shadow, sms, S, cam, Q, L, st); break;
-        case 19: LaunchTraversal<128, 8, MODE_STAGED>(shadow, sms, S, cam, Q, L, st); break;
-        default: LaunchTraversal<128, 8, MODE_LOOP>(shadow, sms, S, cam, Q, L, st); break;
-    }
+    // a tile wave of several scenes and the watertight test have one block count
+    if (Q.scenes && cam.watertight) LaunchTraversal<7, true, true>(shadow, sms, S, cam, Q, L, st);
+    else if (Q.scenes) LaunchTraversal<8, false, true>(shadow, sms, S, cam, Q, L, st);
+    else if (cam.watertight) LaunchTraversal<7, true, false>(shadow, sms, S, cam, Q, L, st);
+    else if (loop) LaunchTraversal<0, false, false>(shadow, sms, S, cam, Q, L, st);
+    else if (kVariants[v].minb == 7) LaunchTraversal<7, false, false>(shadow, sms, S, cam, Q, L, st);
+    else LaunchTraversal<8, false, false>(shadow, sms, S, cam, Q, L, st);
 }
 
 }  // namespace
@@ -863,7 +812,7 @@ static int RenderWave(const GpuScene &G, const CameraParams &cam, WaveBuffers &W
             AZ_CUDA_TRY(cudaEventRecord(W.ev_join, W.side));
             if (L < levels) LaunchTraversalVariant(v, false, sms, D, cam, Q, L + 1, st);
             AZ_CUDA_TRY(cudaStreamWaitEvent(st, W.ev_join, 0));
-            rc.launches += D.full_light_queries ? 4 : 3;
+            rc.launches += 3 + D.full_light_queries + D.entity_lights;
             rc.extend_launches++;
         }
     }
@@ -888,7 +837,7 @@ static int RenderWave(const GpuScene &G, const CameraParams &cam, WaveBuffers &W
         }
         LaunchTraversalVariant(cam.shadow_variant, true, sms, D, cam, Q, L, st);
         if (timer) timer->Mark(st, 3);
-        rc.launches += D.full_light_queries ? 4 : 3;
+        rc.launches += 3 + D.full_light_queries + D.entity_lights;
         rc.extend_launches++;
     }
     if (guide && train) {
@@ -958,6 +907,36 @@ static int ReplayWave(const GpuScene &G, const CameraParams &cam, WaveBuffers &W
     return AZ_OK;
 }
 
+void ChooseDefaultVariants(GpuScene &G) {
+    constexpr uint32_t kLoop = 10, kTogether = 9, kEight = 7, kTwelve = 3;   // {0, 32}, {8, 32}, {8, 8}, {8, 12}
+    // Scenes of a few nodes (Cornell box 1 + 1, 1 M samples: 1.61 ms a frame
+    // with one query per thread, 1.82 by phases).  The visibility queries of
+    // several kinds of light take different paths in a warp all the same (the
+    // features scene, six lights: 6.2 ms one per thread, 3.9 by phases).
+    if (G.node_count <= 64) {
+        G.variant = kLoop;
+        G.shadow_variant = G.dev.light_count + (G.dev.use_env_map ? 1u : 0u) <= 2 ? kLoop : kTogether;
+        return;
+    }
+    // Larger hierarchies (dense mesh / interior / moving spheres, full frames,
+    // with 6, 8, 10 and 14 waiting lanes): closest hits 91 / 170 / 114,
+    // 89 / 170 / 115, 88 / 171 / 117, 89 / 178 / 120 ms; visibility with 6, 10
+    // and 14: 69 / 65 / 19.6, 66 / 67 / 20.2, 64 / 69 / 21.1 ms.
+    G.variant = kEight;
+    G.shadow_variant = kTwelve;
+}
+
+// The launch configurations of a render: the one the caller names (for both
+// traversal kernels), else the scene's.
+static int ChooseVariants(const GpuScene &G, const az_render_opts *opts, CameraParams &cam) {
+    cam.variant = opts && opts->variant ? opts->variant - 1 : G.variant;
+    if (cam.variant >= kVariantCount) return SetError(AZ_ERR_INVALID_ARGUMENT, "unknown launch variant");
+    cam.shadow_variant = (opts && opts->variant) || G.shadow_variant >= kVariantCount ? cam.variant : G.shadow_variant;
+    cam.refill = kVariants[cam.variant].refill;
+    cam.shadow_refill = kVariants[cam.shadow_variant].refill;
+    return AZ_OK;
+}
+
 // The queue ordering of a render: the flags', else the scene's choice.
 static uint32_t QueueOrder(const GpuScene &G, const az_render_opts *opts) {
     const uint32_t f = opts ? opts->flags : 0u;
@@ -1000,10 +979,7 @@ int Render(GpuScene &G, az_pixel *film, const az_camera *camera, const az_epsilo
     cam.sample_out = sample_out;
     cam.count_traversal = opts && (opts->flags & AZ_FLAG_COUNT_TRAVERSAL) ? 1u : 0u;
     cam.env_importance = opts && (opts->flags & AZ_FLAG_ENV_IMPORTANCE) && G.dev.env_rows ? 1u : 0u;
-    cam.variant = opts && opts->variant ? opts->variant - 1 : G.variant;
-    if (cam.variant >= kVariantCount) return SetError(AZ_ERR_INVALID_ARGUMENT, "unknown launch variant");
-    // a variant the caller names applies to both traversal kernels
-    cam.shadow_variant = (opts && opts->variant) || G.shadow_variant >= kVariantCount ? cam.variant : G.shadow_variant;
+    if ((rc = ChooseVariants(G, opts, cam)) != AZ_OK) return rc;
     cam.order = QueueOrder(G, opts);
     cam.serial_levels = opts && (opts->flags & AZ_FLAG_SERIAL_LEVELS) ? 1u : 0u;
     cam.watertight = opts && (opts->flags & AZ_FLAG_WATERTIGHT) ? 1u : 0u;
@@ -1146,6 +1122,7 @@ int RenderTiles(GpuScene &G, std::vector<TileJob> &jobs, const az_render_opts *o
         if (d.max_depth + 1 > AZ_MAX_LEVELS - 2) return SetError(AZ_ERR_UNSUPPORTED, "MaxRecursionDepth above 61");
         wave_dev.features |= d.features;
         wave_dev.full_light_queries |= d.full_light_queries;
+        wave_dev.entity_lights |= d.entity_lights;
         wave_dev.top_spheres += d.top_spheres;
         wave_dev.max_depth = std::max(wave_dev.max_depth, d.max_depth);
         per_node_shadow = std::max(per_node_shadow, d.light_count + (d.use_env_map ? 1u : 0u));
@@ -1162,9 +1139,7 @@ int RenderTiles(GpuScene &G, std::vector<TileJob> &jobs, const az_render_opts *o
         c.scene = scene_of[j];
         c.count_traversal = opts && (opts->flags & AZ_FLAG_COUNT_TRAVERSAL) ? 1u : 0u;
         c.env_importance = opts && (opts->flags & AZ_FLAG_ENV_IMPORTANCE) && Gj.dev.env_rows ? 1u : 0u;
-        c.variant = opts && opts->variant ? opts->variant - 1 : G.variant;
-        if (c.variant >= kVariantCount) return SetError(AZ_ERR_INVALID_ARGUMENT, "unknown launch variant");
-        c.shadow_variant = (opts && opts->variant) || G.shadow_variant >= kVariantCount ? c.variant : G.shadow_variant;
+        if ((rc = ChooseVariants(G, opts, c)) != AZ_OK) return rc;
         // several scenes: no queue ordering (its keys use one scene's bounds)
         c.order = multi ? 0u : QueueOrder(G, opts);
         c.serial_levels = opts && (opts->flags & AZ_FLAG_SERIAL_LEVELS) ? 1u : 0u;
@@ -1540,10 +1515,7 @@ extern "C" int az_gpu_render_noalloc(az_gpu_scene *scene, az_pixel *film, const 
     CameraParams cam;
     rc = SetupCamera(camera, scissor, filter_type, backface_culling, epsilons, opts ? opts->seed : 0, cam);
     if (rc != AZ_OK) return rc;
-    cam.variant = opts && opts->variant ? opts->variant - 1 : G.variant;
-    if (cam.variant >= kVariantCount) return SetError(AZ_ERR_INVALID_ARGUMENT, "unknown launch variant");
-    // a variant the caller names applies to both traversal kernels
-    cam.shadow_variant = (opts && opts->variant) || G.shadow_variant >= kVariantCount ? cam.variant : G.shadow_variant;
+    if ((rc = ChooseVariants(G, opts, cam)) != AZ_OK) return rc;
     // flags whose work would need buffers of their own or a statistics output
     const uint32_t flags = opts ? opts->flags : 0u;
     const uint32_t refused = AZ_FLAG_COUNT_TRAVERSAL | AZ_FLAG_TIME_STAGES | AZ_FLAG_ORDER_SHADOW | AZ_FLAG_ORDER_EXTEND;

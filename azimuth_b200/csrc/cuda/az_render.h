@@ -46,6 +46,7 @@ struct CameraParams {
                                    // with the next level's closest-hit queries
     uint32_t watertight;           // AZ_FLAG_WATERTIGHT: triangles by the watertight test
     uint32_t scene;                // a tile wave of several scenes: the job's index in WaveQueues.scenes
+    uint32_t refill, shadow_refill;   // lanes of a traversal warp that take new queries together (kVariants)
     float4 *sample_out;            // per-sample radiance output (az_gpu_render_samples): sample s of the
                                    // scissor at [s] instead of a splat into the film; null: splat
 };

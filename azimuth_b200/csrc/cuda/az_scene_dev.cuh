@@ -186,6 +186,7 @@ struct DevScene {
     uint32_t light_draws;           // RNG draws made by the light loop at every vertex
     uint32_t features;              // FEAT_* bits
     uint32_t full_light_queries;    // 1: an entity light needs full nearest-hit visibility queries
+    uint32_t entity_lights;         // 1: an entity light does not (its queries' limits: k_light_limits)
     uint32_t top_spheres;           // sphere entities at the top level (the traversal kernels with the
                                     // sphere test inline serve scenes that have any)
     // luminance CDF of a 2D environment map (null when the scene has none):

@@ -915,16 +915,18 @@ int BuildGpuScene(const az_scene *scene, const az_render_opts *opts, cudaStream_
     if (scene->UseEnvironmentMap) D.features |= azd::FEAT_ENV;
     for (const azd::DevMaterial &m : mats)
         if (m.transparent || m.is_mirror) D.features |= azd::FEAT_SPECIAL;
-    D.full_light_queries = 0;
+    D.full_light_queries = D.entity_lights = 0;
     D.top_spheres = (uint32_t)(tlas.size() - dgroups.size());
     for (const azd::DevLight &l : lights) {
         if (l.type != azd::LIGHT_ENTITY) D.features |= azd::FEAT_ANALYTIC_LIGHTS;
         else if (azd::entity_light_needs_full_query(l)) D.full_light_queries = 1;
+        else D.entity_lights = 1;
     }
     AZ_CUDA_TRY(cudaStreamSynchronize(st));
     G->triangle_count = total_tris;
     G->sphere_count = tlas.size() - dgroups.size();
     G->node_count = wide_count;
+    ChooseDefaultVariants(*G);
     G->max_bvh_depth = wide_depth;
     G->total_ms = std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t_start).count();
     *out = G.release();

@@ -424,21 +424,6 @@ static __device__ void sample_entity_light(const DevScene &S, const DevLight &L,
 // `triangle` array, whose vertices are the triangle entities' vertices).
 // Returns 1 with the world t, 0 if the light is not hit, -1 if the light
 // needs a full nearest-hit query instead (entity_light_needs_full_query).
-// Called out of line by the visibility kernels (values and global pointers
-// only), which keeps their traversal loop small.
-struct LightHit {
-    int hit;
-    float t;   // world t when hit; FLT_MAX otherwise
-};
-static __device__ int light_entity_hit(const DevEntity *ents, const DevLightTri *light_tris, const DevLight &L,
-                                       const Ray &wr, float &t_world);
-static __device__ __noinline__ LightHit light_entity_hit_call(const DevEntity *ents, const DevLightTri *light_tris,
-                                                             const DevLight *L, Ray wr) {
-    LightHit h;
-    h.t = FLT_MAX;
-    h.hit = light_entity_hit(ents, light_tris, *L, wr, h.t);
-    return h;
-}
 static __device__ int light_entity_hit(const DevEntity *ents, const DevLightTri *light_tris, const DevLight &L,
                                        const Ray &wr, float &t_world) {
     if (entity_light_needs_full_query(L)) return -1;

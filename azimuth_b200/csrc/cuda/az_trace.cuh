@@ -348,26 +348,12 @@ __device__ __forceinline__ float group_t_scale(const DevGroup &g, f3 d) {
     return length(vector_xf(g.inv, d)) / length(d) * 1.0001f;
 }
 
-// The traversal loops call the rarely taken paths below out of line, with
-// values and global pointers only, so that the loops' own code stays small
-// (the instruction cache of an SM holds the hot loop; a scene's spheres,
-// transformed instances and entity lights take these calls).
-
-// sphere_test of entity e for the world ray: out of line, or inline (INL)
-// in the kernels that serve scenes with spheres at the top level.
+// sphere_test of entity e for the world ray.
 struct SphereHit {
     float t_world, t_local;
     uint32_t hit;
 };
-static __device__ __noinline__ SphereHit sphere_test_call(const DevEntity *e, Ray wr, float eps) {
-    SphereHit h;
-    h.t_world = h.t_local = FLT_MAX;
-    h.hit = sphere_test(*e, wr, eps, h.t_world, h.t_local) ? 1u : 0u;
-    return h;
-}
-template <bool INL>
 __device__ __forceinline__ SphereHit sphere_hit(const DevEntity *e, const Ray &wr, float eps) {
-    if (!INL) return sphere_test_call(e, wr, eps);
     SphereHit h;
     h.t_world = h.t_local = FLT_MAX;
     h.hit = sphere_test(*e, wr, eps, h.t_world, h.t_local) ? 1u : 0u;
@@ -375,7 +361,9 @@ __device__ __forceinline__ SphereHit sphere_hit(const DevEntity *e, const Ray &w
 }
 
 // The local ray of a transformed, possibly moving group (GetLocalRay of the
-// motion-shifted ray) and the group_t_scale of the world direction.
+// motion-shifted ray) and the group_t_scale of the world direction.  Called
+// out of line by the traversal loops, with values and a global pointer only, so
+// that their own code stays small (the instruction cache holds the hot loop).
 struct GroupRay {
     Ray r;
     float scale;
@@ -395,9 +383,7 @@ static __device__ __noinline__ GroupRay group_ray_call(const DevGroup *gp, Ray w
 // Traversal on GPUs Through Compressed Wide BVHs" (HPG 2017): each step
 // visits the nearest node of the current group, then tests the primitives its
 // leaves hit, postponing them onto the stack while few lanes of the warp have
-// primitives to test.  The traversal is a resumable state machine (init, then
-// step() until it reports the query finished) so that persistent kernels can
-// hand a lane a new ray as soon as its query ends.
+// primitives to test.
 //
 // Q_CLOSEST: nearest hit in `best` (best.ent == 0xFFFFFFFF: none).
 // Q_ANY: `hit_any` is set as soon as a primitive's world t < tmax.
@@ -406,312 +392,8 @@ template <QueryKind KIND, bool WT = false>
 __device__ bool trace(const DevScene &S, const Ray &wr, bool cull, float eps, float tmax, Hit &best,
                       uint32_t *counts = nullptr, uint32_t *err = nullptr, uint32_t skip_ent = 0xFFFFFFFFu);
 
-// POP_FIRST: a step that starts with both current groups empty pops the
-// stack until it holds a node or primitive group and visits it in the same
-// step (a finished query is reported at the end of its last step); otherwise
-// a step ends with the pop and the popped group waits for the next step.
-// WT: triangles by the watertight test instead of azimuth's Cramer test.
-// SPH: the top-level sphere test inline (scenes with spheres at the top
-// level); otherwise it is called out of line.
-template <QueryKind KIND, bool POP_FIRST = false, bool WT = false, bool SPH = false>
-struct Tracer {
-    static constexpr uint32_t kNoNode = 0xFFFFFFFFu;
-    Ray wr;                    // world ray
-    Ray r;                     // ray in the current space (world or a group's local space)
-    f3 inv;
-    uint32_t oct;
-    float tcur;                // pruning distance in the current space
-    float tmax, eps;
-    bool cull, in_blas, hit_any;
-    uint32_t skip_ent, g_idx;
-    float bl_t;                // nearest local hit of this BLAS visit
-    uint32_t bl_prim;
-    uint32_t ng_base, ng_bits; // current node group
-    uint32_t pg_base, pg_mask; // current primitive group
-    uint32_t steps, nodes_visited, prims_visited;
-    int sp;
-    Hit best;
-    WtRay wt;                  // WT: shear of the current ray space
-
-    // `stack`: the query's stack (AZD_WSTACK entries), which a scene whose top
-    // level is a single group starts with that group's exit marker.
-    __device__ __forceinline__ void init(const DevScene &S, const Ray &ray, bool cull_, float eps_, float tmax_,
-                                         uint2 *stack, uint32_t skip = 0xFFFFFFFFu) {
-        wr = ray;
-        r = ray;
-        tmax = tmax_;
-        eps = eps_;
-        cull = cull_;
-        tcur = KIND == Q_ANY ? tmax_ : FLT_MAX;
-        in_blas = false;
-        hit_any = false;
-        skip_ent = skip;
-        g_idx = 0;
-        bl_t = FLT_MAX;
-        bl_prim = 0xFFFFFFFFu;
-        pg_base = 0;
-        pg_mask = 0;
-        steps = nodes_visited = prims_visited = 0;
-        sp = 0;
-        best.t = FLT_MAX;
-        best.tl = 0.0f;
-        best.prim = 0xFFFFFFFFu;
-        best.ent = 0xFFFFFFFFu;
-        if (S.tlas_single_group != 0xFFFFFFFFu) {
-            // a top level holding one group only: enter its hierarchy directly
-            // (the top-level root test and the group's leaf would only lead there)
-            inv = mk(0.0f, 0.0f, 0.0f);
-            oct = 0u;
-            ng_base = 0u;
-            ng_bits = 0u;
-            enter_group(S, stack, S.tlas_single_group);
-        } else {
-            // current node group: the root alone (imask bit 0, hit bit 0 ^ oct)
-            inv = safe_inv(r.d);
-            oct = octant_of(r.d);
-            if (WT) wt = wt_setup(r.d);
-            ng_base = S.tlas_root;
-            ng_bits = S.tlas_root == 0xFFFFFFFFu ? 0u : ((1u << 8) | (1u << oct));
-        }
-    }
-
-    // Enters group gi's bottom-level hierarchy (azimuth: GetLocalRay of the
-    // motion-shifted ray, src/azimuth_main.cpp:246-250); its exit marker goes on
-    // the stack (room for it is kept when a group entry is pushed).
-    __device__ __forceinline__ void enter_group(const DevScene &S, uint2 *stack, uint32_t gi) {
-        g_idx = gi;
-        const DevGroup &g = S.groups[g_idx];
-        if (g.root == 0xFFFFFFFFu) return;
-        stack[sp++] = make_uint2(0u, AZD_E_EXIT);
-        const float wlim = KIND == Q_ANY ? tmax : best.t;
-        tcur = FLT_MAX;
-        if (g.raw) {
-            r = wr;
-            if (wlim < FLT_MAX) tcur = wlim + 1e-30f;
-        } else if (g.identity) {
-            r = local_ray_identity(wr);
-            if (wlim < FLT_MAX) tcur = wlim * 1.0001f + 1e-30f;
-        } else {
-            const GroupRay gr = group_ray_call(S.groups + g_idx, wr);
-            r = gr.r;
-            if (wlim < FLT_MAX) tcur = wlim * gr.scale + 1e-30f;
-        }
-        inv = safe_inv(r.d);
-        oct = octant_of(r.d);
-        if (WT) wt = wt_setup(r.d);
-        bl_t = FLT_MAX;
-        bl_prim = 0xFFFFFFFFu;
-        in_blas = true;
-        ng_base = g.root;
-        ng_bits = (1u << 8) | (1u << oct);
-    }
-
-    __device__ __forceinline__ void push(uint2 *stack, uint32_t x, uint32_t y, uint32_t *err) {
-        if (sp < AZD_WSTACK) stack[sp++] = make_uint2(x, y);
-        else if (err) atomicOr(err, 2u);
-    }
-
-    // Takes the top stack entry: leaves or enters a bottom-level hierarchy, or
-    // makes the entry the current primitive or node group.
-    __device__ __forceinline__ void pop(const DevScene &S, uint2 *stack) {
-        const uint2 e = stack[--sp];
-        if (e.y == AZD_E_EXIT) {
-            // leaving a BLAS: azimuth's instance path keeps the nearest local hit
-            // and recomputes its world t (src/azimuth_main.cpp:256-276)
-            if (KIND == Q_CLOSEST && bl_prim != 0xFFFFFFFFu) {
-                float wt_ = group_world_t(S.groups[g_idx], wr, r, bl_t);
-                if (wt_ > eps && wt_ < best.t) {
-                    best.t = wt_;
-                    best.tl = bl_t;
-                    best.prim = bl_prim;
-                    best.ent = S.tri_attr[bl_prim].entity;
-                }
-            }
-            in_blas = false;
-            if (sp == 0) return;   // the query is done: no world-space traversal follows
-            r = wr;
-            inv = safe_inv(r.d);
-            oct = octant_of(r.d);
-            if (WT) wt = wt_setup(r.d);
-            tcur = KIND == Q_ANY ? tmax : best.t;
-        } else if (e.y == AZD_E_GROUP) {
-            enter_group(S, stack, e.x);   // its exit marker reuses the popped entry's slot
-        } else if ((e.y & 0xC0000000u) == AZD_E_PRIMS) {
-            pg_base = e.x;
-            pg_mask = e.y & 0x00FFFFFFu;
-        } else {
-            ng_base = e.x;
-            ng_bits = e.y;
-        }
-    }
-
-    // One step: visit the nearest node of the current group and test the
-    // primitives it hits, and pop the stack when both groups are empty.
-    // Returns true when finished.  The stack (AZD_WSTACK entries) is a
-    // separate array of the caller so that the state above stays in registers.
-    __device__ __forceinline__ bool step(const DevScene &S, uint2 *stack, uint32_t *err) {
-        uint32_t node;
-        if (begin(S, stack, err, node)) return true;
-        uint4 w[5];
-        if (node != kNoNode) {
-            const uint4 *np = reinterpret_cast<const uint4 *>(S.wnodes + node);
-#pragma unroll
-            for (int k = 0; k < 5; k++) w[k] = __ldg(np + k);
-        }
-        return finish(S, stack, err, node, w);
-    }
-
-    // The first half of a step: the step count, the pops of a pop-first
-    // tracer, and the choice of the node to visit (`node`, kNoNode when the
-    // step visits none).  Returns true when the query is finished.  A caller
-    // that fetches the node itself (stage_nodes) runs begin, the fetch, then
-    // finish.
-    __device__ __forceinline__ bool begin(const DevScene &S, uint2 *stack, uint32_t *err, uint32_t &node) {
-        node = kNoNode;
-        if (++steps > AZD_MAX_STEPS) {
-            if (err) atomicOr(err, 1u);
-            return true;
-        }
-        if (POP_FIRST) {
-            while (!(ng_bits & 0xFFu) && !pg_mask) {
-                if (sp == 0) return true;
-                pop(S, stack);
-            }
-        }
-        if (ng_bits & 0xFFu) {
-            const uint32_t hits = ng_bits & 0xFFu, imask = (ng_bits >> 8) & 0xFFu;
-            const uint32_t key = child_key<KIND>(hits);
-            const uint32_t slot = key ^ oct;
-            node = ng_base + __popc(imask & ((1u << slot) - 1u));
-            ng_bits &= ~(1u << key);
-            if (ng_bits & 0xFFu) push(stack, ng_base, ng_bits, err);
-        }
-        return false;
-    }
-
-    // The second half: the eight child tests of `node` (w: its five 16-byte
-    // words), the primitives, and the pop of exhausted groups.  Returns true
-    // when the query is finished.
-    __device__ __forceinline__ bool finish(const DevScene &S, uint2 *stack, uint32_t *err, uint32_t node,
-                                           const uint4 (&w)[5]) {
-        if (node != kNoNode) {
-            nodes_visited++;
-            const WideHits h = wide_test(w[0], w[1], w[2], w[3], w[4], r.o, inv, oct, tcur);
-            ng_base = w[1].x;
-            ng_bits = h.inner | ((w[0].w >> 24) << 8);
-            if (h.prims) {
-                if (pg_mask) push(stack, pg_base, AZD_E_PRIMS | pg_mask, err);   // keep the older group for later
-                pg_base = w[1].y;
-                pg_mask = h.prims;
-            }
-        }
-        // primitives, postponed while few lanes of the warp have any
-        while (pg_mask) {
-            if (__popc(__activemask()) < 6u && (ng_bits & 0xFFu) && sp < AZD_WSTACK) {
-                stack[sp++] = make_uint2(pg_base, AZD_E_PRIMS | pg_mask);
-                pg_mask = 0;
-                break;
-            }
-            const uint32_t bit = __ffs(pg_mask) - 1u;
-            pg_mask &= pg_mask - 1u;
-            const uint32_t pi = pg_base + bit;
-            prims_visited++;
-            if (in_blas) {
-                float t, b, gm;
-                bool hit;
-                if (WT) {
-                    hit = tri_test_wt(load_tri_verts(S.tri_verts, pi), r, wt, cull, eps, bl_t, t);
-                } else {
-                    hit = tri_test(load_tri(S.tris, pi), r, cull, eps, bl_t, t, b, gm);
-                }
-                if (hit) {
-                    // a primitive of the skipped entity is ignored; its owner is
-                    // looked up only for the few primitives that are hit
-                    if (skip_ent != 0xFFFFFFFFu && __ldg(&S.tri_attr[pi].entity) == skip_ent) continue;
-                    bl_t = t;
-                    bl_prim = pi;
-                    if (KIND == Q_ANY) {
-                        // finished as soon as one hit of this group is in range
-                        float wt = group_world_t(S.groups[g_idx], wr, r, t);
-                        if (wt > eps && wt < tmax) {
-                            hit_any = true;
-                            return true;
-                        }
-                    } else {
-                        tcur = fminf(tcur, t);
-                    }
-                }
-            } else {
-                const uint32_t p = __ldg(S.tlas_prims + pi);
-                if (p & AZD_TLAS_GROUP) {
-                    push(stack, p & ~AZD_TLAS_GROUP, AZD_E_GROUP, err);   // entered when popped
-                } else if (p != skip_ent && S.ents[p].type == ENT_SPHERE) {
-                    const SphereHit sh = sphere_hit<SPH>(S.ents + p, wr, eps);
-                    if (sh.hit) {
-                        if (KIND == Q_ANY) {
-                            if (sh.t_world < tmax) {
-                                hit_any = true;
-                                return true;
-                            }
-                        } else if (sh.t_world < best.t) {
-                            best.t = sh.t_world;
-                            best.tl = sh.t_local;
-                            best.prim = 0xFFFFFFFFu;
-                            best.ent = p;
-                            tcur = sh.t_world;
-                        }
-                    }
-                }
-            }
-        }
-        if ((ng_bits & 0xFFu) || pg_mask) return false;
-        // nothing left in the current groups: pop (or, popping first, let the
-        // next step pop; a leftover BLAS exit marker must still be taken)
-        if (sp == 0) return true;
-        if (POP_FIRST) return false;
-        pop(S, stack);
-        return false;
-    }
-
-    __device__ __forceinline__ void flush_counts(uint32_t *counts) const {
-        if (counts) {
-            atomicAdd(counts + 0, nodes_visited);
-            atomicAdd(counts + 1, prims_visited);
-        }
-    }
-};
-
-// Node fetch staged through shared memory, called by all 32 lanes of a warp
-// between Tracer::begin and Tracer::finish.  The nodes that the lanes visit
-// this step (node: kNoNode for none) are loaded together: 16-byte word c of
-// the warp's list (word c % 5 of lane c / 5's node) is read by lane c % 32 in
-// round c / 32, so five neighbouring lanes read one node's 80 contiguous bytes
-// instead of every lane reading 16 bytes of its own node per instruction;
-// each lane then takes its node's five words from `stage` (the warp's 160
-// words of shared memory).
-__device__ __forceinline__ void stage_nodes(const WideNode *nodes, uint32_t node, uint4 *stage, uint4 (&w)[5]) {
-    constexpr uint32_t kNone = 0xFFFFFFFFu;
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t want = __ballot_sync(0xFFFFFFFFu, node != kNone);
-    if (!want) return;
-    const uint4 *base = reinterpret_cast<const uint4 *>(nodes);
-#pragma unroll
-    for (uint32_t it = 0; it < 5; it++) {
-        const uint32_t c = 32u * it + lane, j = c / 5u, part = c - 5u * j;
-        const uint32_t nj = __shfl_sync(0xFFFFFFFFu, node, j);
-        if ((want >> j) & 1u) stage[c] = __ldg(base + (size_t)nj * 5u + part);
-    }
-    __syncwarp();
-    if (node != kNone) {
-#pragma unroll
-        for (int k = 0; k < 5; k++) w[k] = stage[5u * lane + k];
-    }
-    __syncwarp();   // the stage is free for the next step
-}
-
-// A whole query in one loop: the same traversal as Tracer written as a single
-// function, which the compiler schedules better when one thread runs one
-// query to its end (grid-stride kernels).  For Q_CLOSEST returns whether
+// A whole query run by one thread to its end (single queries and the rare full
+// nearest-hit light queries; the wave's queues are traced by az_phase.cuh).  For Q_CLOSEST returns whether
 // something was hit and the nearest hit in `best`; for Q_ANY returns whether a
 // primitive lies closer than tmax.  `skip_ent` is an entity whose primitives
 // are ignored; `counts` accumulates node and primitive visits.
@@ -825,7 +507,7 @@ __device__ bool trace(const DevScene &S, const Ray &wr, bool cull, float eps, fl
                     if (sp + 1 < AZD_WSTACK) stack[sp++] = make_uint2(p & ~AZD_TLAS_GROUP, AZD_E_GROUP);
                     else if (err) atomicOr(err, 2u);
                 } else if (p != skip_ent && S.ents[p].type == ENT_SPHERE) {
-                    const SphereHit sh = sphere_hit<true>(S.ents + p, wr, eps);
+                    const SphereHit sh = sphere_hit(S.ents + p, wr, eps);
                     if (sh.hit) {
                         if (KIND == Q_ANY) {
                             if (sh.t_world < tmax) {

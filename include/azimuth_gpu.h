@@ -81,12 +81,11 @@ typedef struct az_render_opts {
                                        scene for its next render */
     uint32_t bvh_width;             /* az_gpu_scene_create: children per BVH node, 2, 4 or 8 (0 = 8) */
     uint32_t block_size;            /* reserved (0) */
-    uint32_t variant;               /* traversal launch configuration 1..AZ_LAUNCH_VARIANTS (threads per
-                                       block, register cap, how queries map to threads: one per thread
-                                       to its end, warp lockstep per traversal step, or persistent
-                                       fetching, with node fetches staged through shared memory in
-                                       variants 19 and 20); 0 = the scene's choice: 8 (128 threads, at most 64
-                                       registers, persistent fetching) until az_gpu_autotune picks another */
+    uint32_t variant;               /* traversal launch configuration 1..AZ_LAUNCH_VARIANTS (register cap,
+                                       how many lanes of a warp wait for each other before they take
+                                       new queries, or one query per thread); 0 = the scene's choice,
+                                       by the size of its hierarchy, until az_gpu_autotune picks
+                                       another */
     uint32_t bvh_leaf;              /* az_gpu_scene_create: triangles per bottom-level leaf at most, 1..3 (0 = 2) */
     uint32_t bvh_builder;           /* az_gpu_scene_create: binary hierarchy before the wide collapse,
                                        AZ_BVH_LBVH or AZ_BVH_PLOC (0 = the default, AZ_BVH_PLOC) */
