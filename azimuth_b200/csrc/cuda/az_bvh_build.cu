@@ -9,6 +9,7 @@
 #include <cfloat>
 
 #include "az_internal.h"
+#include "az_pool.h"
 
 namespace az {
 namespace {
@@ -198,15 +199,6 @@ __global__ void k_single(const float4 *lo, const float4 *hi, azd::BVHNode *nodes
     perm[0] = 0;
 }
 
-template <typename T>
-struct Scratch {
-    T *p = nullptr;
-    ~Scratch() {
-        if (p) cudaFree(p);
-    }
-    cudaError_t alloc(size_t n) { return cudaMalloc((void **)&p, n * sizeof(T) + 16); }
-};
-
 // ---- PLOC: parallel locally-ordered clustering (Meister, Bittner, "Parallel
 // Locally-Ordered Clustering for Bounding Volume Hierarchy Construction",
 // IEEE TVCG 2018).  The clusters, kept in Morton order, each find the
@@ -373,41 +365,41 @@ __global__ void k_ploc_perm(const uint32_t *order, const uint32_t *leaf_first, u
 int BuildPLOC(const float4 *d_lo, const float4 *d_hi, uint32_t n, azd::BVHNode *d_nodes, uint2 *d_range,
               uint32_t node_base, uint32_t leaf_base, uint32_t *d_perm, cudaStream_t stream, uint32_t *root_out) {
     if (n <= 2) return BuildLBVH(d_lo, d_hi, n, d_nodes, d_range, node_base, leaf_base, d_perm, stream, root_out);
-    Scratch<float> bounds;
-    Scratch<unsigned long long> keys, keys_sorted, flags, incl;
-    Scratch<uint32_t> vals, order, ids_a, ids_b, nn, nl, nr, ncount, nfirst, lfirst;
-    Scratch<float4> lo_a, hi_a, lo_b, hi_b, nlo, nhi;
-    Scratch<unsigned char> temp, temp2;
-    Scratch<uint32_t> err;
-    AZ_CUDA_TRY(err.alloc(1));
+    PoolBuf<float> bounds;
+    PoolBuf<unsigned long long> keys, keys_sorted, flags, incl;
+    PoolBuf<uint32_t> vals, order, ids_a, ids_b, nn, nl, nr, ncount, nfirst, lfirst;
+    PoolBuf<float4> lo_a, hi_a, lo_b, hi_b, nlo, nhi;
+    PoolBuf<unsigned char> temp, temp2;
+    PoolBuf<uint32_t> err;
+    AZ_CUDA_TRY(err.alloc(1, stream));
     AZ_CUDA_TRY(cudaMemsetAsync(err.p, 0, sizeof(uint32_t), stream));
-    AZ_CUDA_TRY(bounds.alloc(6));
-    AZ_CUDA_TRY(keys.alloc(n));
-    AZ_CUDA_TRY(keys_sorted.alloc(n));
-    AZ_CUDA_TRY(vals.alloc(n));
-    AZ_CUDA_TRY(order.alloc(n));
-    AZ_CUDA_TRY(ids_a.alloc(n));
-    AZ_CUDA_TRY(ids_b.alloc(n));
-    AZ_CUDA_TRY(lo_a.alloc(n));
-    AZ_CUDA_TRY(hi_a.alloc(n));
-    AZ_CUDA_TRY(lo_b.alloc(n));
-    AZ_CUDA_TRY(hi_b.alloc(n));
-    AZ_CUDA_TRY(nn.alloc(n));
-    AZ_CUDA_TRY(flags.alloc(n));
-    AZ_CUDA_TRY(incl.alloc(n));
-    AZ_CUDA_TRY(nl.alloc(n));
-    AZ_CUDA_TRY(nr.alloc(n));
-    AZ_CUDA_TRY(nlo.alloc(n));
-    AZ_CUDA_TRY(nhi.alloc(n));
-    AZ_CUDA_TRY(ncount.alloc(n));
-    AZ_CUDA_TRY(nfirst.alloc(n));
-    AZ_CUDA_TRY(lfirst.alloc(n));
+    AZ_CUDA_TRY(bounds.alloc(6, stream));
+    AZ_CUDA_TRY(keys.alloc(n, stream));
+    AZ_CUDA_TRY(keys_sorted.alloc(n, stream));
+    AZ_CUDA_TRY(vals.alloc(n, stream));
+    AZ_CUDA_TRY(order.alloc(n, stream));
+    AZ_CUDA_TRY(ids_a.alloc(n, stream));
+    AZ_CUDA_TRY(ids_b.alloc(n, stream));
+    AZ_CUDA_TRY(lo_a.alloc(n, stream));
+    AZ_CUDA_TRY(hi_a.alloc(n, stream));
+    AZ_CUDA_TRY(lo_b.alloc(n, stream));
+    AZ_CUDA_TRY(hi_b.alloc(n, stream));
+    AZ_CUDA_TRY(nn.alloc(n, stream));
+    AZ_CUDA_TRY(flags.alloc(n, stream));
+    AZ_CUDA_TRY(incl.alloc(n, stream));
+    AZ_CUDA_TRY(nl.alloc(n, stream));
+    AZ_CUDA_TRY(nr.alloc(n, stream));
+    AZ_CUDA_TRY(nlo.alloc(n, stream));
+    AZ_CUDA_TRY(nhi.alloc(n, stream));
+    AZ_CUDA_TRY(ncount.alloc(n, stream));
+    AZ_CUDA_TRY(nfirst.alloc(n, stream));
+    AZ_CUDA_TRY(lfirst.alloc(n, stream));
     size_t temp_bytes = 0, temp2_bytes = 0;
     AZ_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, keys.p, keys_sorted.p, vals.p, order.p, (int)n, 0,
                                                 63, stream));
-    AZ_CUDA_TRY(temp.alloc(temp_bytes));
+    AZ_CUDA_TRY(temp.alloc(temp_bytes, stream));
     AZ_CUDA_TRY(cub::DeviceScan::InclusiveSum(nullptr, temp2_bytes, flags.p, incl.p, (int)n, stream));
-    AZ_CUDA_TRY(temp2.alloc(temp2_bytes));
+    AZ_CUDA_TRY(temp2.alloc(temp2_bytes, stream));
     const int B = 256;
     k_bounds_reduce<<<1, 256, 0, stream>>>(d_lo, d_hi, n, bounds.p);
     k_morton<<<(n + B - 1) / B, B, 0, stream>>>(d_lo, d_hi, n, bounds.p, keys.p, vals.p);
@@ -477,30 +469,30 @@ int BuildLBVH(const float4 *d_lo, const float4 *d_hi, uint32_t n, azd::BVHNode *
         AZ_CUDA_TRY(cudaGetLastError());
         return AZ_OK;
     }
-    Scratch<float> bounds;
-    Scratch<unsigned long long> keys, keys_sorted;
-    Scratch<uint32_t> vals, vals_sorted;
-    Scratch<uint32_t> left, right;
-    Scratch<int> parent_int, parent_leaf;
-    Scratch<float4> ilo, ihi;
-    Scratch<unsigned int> visits;
-    Scratch<unsigned char> temp;
-    AZ_CUDA_TRY(bounds.alloc(6));
-    AZ_CUDA_TRY(keys.alloc(n));
-    AZ_CUDA_TRY(keys_sorted.alloc(n));
-    AZ_CUDA_TRY(vals.alloc(n));
-    AZ_CUDA_TRY(vals_sorted.alloc(n));
-    AZ_CUDA_TRY(left.alloc(n));
-    AZ_CUDA_TRY(right.alloc(n));
-    AZ_CUDA_TRY(parent_int.alloc(n));
-    AZ_CUDA_TRY(parent_leaf.alloc(n));
-    AZ_CUDA_TRY(ilo.alloc(n));
-    AZ_CUDA_TRY(ihi.alloc(n));
-    AZ_CUDA_TRY(visits.alloc(n));
+    PoolBuf<float> bounds;
+    PoolBuf<unsigned long long> keys, keys_sorted;
+    PoolBuf<uint32_t> vals, vals_sorted;
+    PoolBuf<uint32_t> left, right;
+    PoolBuf<int> parent_int, parent_leaf;
+    PoolBuf<float4> ilo, ihi;
+    PoolBuf<unsigned int> visits;
+    PoolBuf<unsigned char> temp;
+    AZ_CUDA_TRY(bounds.alloc(6, stream));
+    AZ_CUDA_TRY(keys.alloc(n, stream));
+    AZ_CUDA_TRY(keys_sorted.alloc(n, stream));
+    AZ_CUDA_TRY(vals.alloc(n, stream));
+    AZ_CUDA_TRY(vals_sorted.alloc(n, stream));
+    AZ_CUDA_TRY(left.alloc(n, stream));
+    AZ_CUDA_TRY(right.alloc(n, stream));
+    AZ_CUDA_TRY(parent_int.alloc(n, stream));
+    AZ_CUDA_TRY(parent_leaf.alloc(n, stream));
+    AZ_CUDA_TRY(ilo.alloc(n, stream));
+    AZ_CUDA_TRY(ihi.alloc(n, stream));
+    AZ_CUDA_TRY(visits.alloc(n, stream));
     size_t temp_bytes = 0;
     AZ_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, keys.p, keys_sorted.p, vals.p, vals_sorted.p,
                                                 (int)n, 0, 63, stream));
-    AZ_CUDA_TRY(temp.alloc(temp_bytes));
+    AZ_CUDA_TRY(temp.alloc(temp_bytes, stream));
     const int B = 256;
     uint32_t grid = (n + B - 1) / B;
     k_bounds_reduce<<<1, 256, 0, stream>>>(d_lo, d_hi, n, bounds.p);

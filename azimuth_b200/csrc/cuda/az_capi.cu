@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "az_internal.h"
+#include "az_pool.h"
 #include "azimuth_io.h"
 
 namespace az {
@@ -49,16 +50,13 @@ struct CallContext {
         } else {
             // a blocking stream: ordered after earlier work on the legacy default
             // stream (a film zeroed there, for instance)
-            AZ_CUDA_TRY(cudaStreamCreate(&stream));
+            AZ_CUDA_TRY(AcquireStream(&stream));
             own = true;
         }
         return AZ_OK;
     }
     ~CallContext() {
-        if (own && stream) {
-            cudaStreamSynchronize(stream);
-            cudaStreamDestroy(stream);
-        }
+        if (own && stream) ReleaseStream(stream);
     }
 };
 
@@ -228,10 +226,10 @@ extern "C" int az_gpu_render_host(az_gpu_scene *scene, az_pixel *pixels, const a
     GpuScene &G = *scene->impl;
     size_t bytes = (size_t)camera->Resolution.x * camera->Resolution.y * sizeof(az_pixel);
     if (G.host_film_bytes < bytes) {
-        if (G.host_film_dev) cudaFree(G.host_film_dev);
+        PoolFree(G.host_film_dev, ctx.stream);
         G.host_film_dev = nullptr;
         G.host_film_bytes = 0;
-        AZ_CUDA_TRY(cudaMalloc((void **)&G.host_film_dev, bytes));
+        AZ_CUDA_TRY(PoolAlloc((void **)&G.host_film_dev, bytes, ctx.stream));
         G.host_film_bytes = bytes;
     }
     AZ_CUDA_TRY(cudaMemcpyAsync(G.host_film_dev, pixels, bytes, cudaMemcpyHostToDevice, ctx.stream));
@@ -255,22 +253,18 @@ extern "C" int az_gpu_produce_image(az_pixel *pixels, const az_scene *scene, con
     if (rc != AZ_OK) return rc;
     std::unique_ptr<GpuScene> hold(g);
     size_t bytes = (size_t)camera->Resolution.x * camera->Resolution.y * sizeof(az_pixel);
-    az_pixel *d_film = nullptr;
-    AZ_CUDA_TRY(cudaMallocAsync((void **)&d_film, bytes, ctx.stream));
+    PoolBuf<unsigned char> film;
+    AZ_CUDA_TRY(film.alloc(bytes, ctx.stream));
+    az_pixel *d_film = (az_pixel *)film.p;
     // the film accumulates: start from the caller's sums
     cudaError_t e = cudaMemcpyAsync(d_film, pixels, bytes, cudaMemcpyHostToDevice, ctx.stream);
-    if (e != cudaSuccess) {
-        cudaFreeAsync(d_film, ctx.stream);
-        return CudaError(e, "film upload");
-    }
+    if (e != cudaSuccess) return CudaError(e, "film upload");
     rc = Render(*g, d_film, camera, epsilons, scissor, filter_type, backface_culling, opts, ctx.stream, nullptr);
     if (rc == AZ_OK) {
         e = cudaMemcpyAsync(pixels, d_film, bytes, cudaMemcpyDeviceToHost, ctx.stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx.stream);
         if (e != cudaSuccess) rc = CudaError(e, "film download");
     }
-    cudaFreeAsync(d_film, ctx.stream);
-    cudaStreamSynchronize(ctx.stream);
     return rc;
 }
 
@@ -393,15 +387,14 @@ extern "C" int az_gpu_output_pixels_to_file(const char *path, const az_pixel *fi
             exr_path = az_exr_sibling_path(path, sib, sizeof(sib)) == AZ_OK ? std::string(sib) : std::string();
         }
         if (!exr_path.empty()) {
-            float *d_rgb = nullptr;
-            AZ_CUDA_TRY(cudaMalloc((void **)&d_rgb, n * 3 * sizeof(float)));
-            rc = PostProcess(film, width, height, tonemap, inv_gamma, srgb, 1, d_rgb, nullptr, ctx.stream);
+            PoolBuf<float> d_rgb;
+            AZ_CUDA_TRY(d_rgb.alloc(n * 3, ctx.stream));
+            rc = PostProcess(film, width, height, tonemap, inv_gamma, srgb, 1, d_rgb.p, nullptr, ctx.stream);
             std::vector<float> rgb(n * 3);
             if (rc == AZ_OK) {
-                cudaError_t e = cudaMemcpy(rgb.data(), d_rgb, n * 3 * sizeof(float), cudaMemcpyDeviceToHost);
+                cudaError_t e = cudaMemcpy(rgb.data(), d_rgb.p, n * 3 * sizeof(float), cudaMemcpyDeviceToHost);
                 if (e != cudaSuccess) rc = CudaError(e, "cudaMemcpy(EXR colours)");
             }
-            cudaFree(d_rgb);
             if (rc != AZ_OK) return rc;
             for (float &c : rgb) c = c * 255.0f;
             if (az_write_exr(exr_path.c_str(), rgb.data(), width, height) != AZ_OK)
@@ -409,15 +402,14 @@ extern "C" int az_gpu_output_pixels_to_file(const char *path, const az_pixel *fi
         }
         if (format == AZ_FileFormat_EXR) return AZ_OK;
     }
-    uint8_t *d_rgb8 = nullptr;
-    AZ_CUDA_TRY(cudaMalloc((void **)&d_rgb8, n * 3));
-    rc = PostProcess(film, width, height, tonemap, inv_gamma, srgb, 0, nullptr, d_rgb8, ctx.stream);
+    PoolBuf<uint8_t> d_rgb8;
+    AZ_CUDA_TRY(d_rgb8.alloc(n * 3, ctx.stream));
+    rc = PostProcess(film, width, height, tonemap, inv_gamma, srgb, 0, nullptr, d_rgb8.p, ctx.stream);
     std::vector<uint8_t> rgb8(n * 3);
     if (rc == AZ_OK) {
-        cudaError_t e = cudaMemcpy(rgb8.data(), d_rgb8, n * 3, cudaMemcpyDeviceToHost);
+        cudaError_t e = cudaMemcpy(rgb8.data(), d_rgb8.p, n * 3, cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) rc = CudaError(e, "cudaMemcpy(8-bit colours)");
     }
-    cudaFree(d_rgb8);
     if (rc != AZ_OK) return rc;
     if (az_write_image(path, rgb8.data(), width, height, format) != AZ_OK)
         return SetError(AZ_ERR_IO, std::string("cannot write ") + path);

@@ -29,6 +29,7 @@
 
 #include "az_guide.cuh"
 #include "az_internal.h"
+#include "az_pool.h"
 #include "az_render.h"
 #include "az_shade.cuh"
 #include "azimuth_gpu.h"
@@ -1508,10 +1509,10 @@ void DestroyGuide(GuideState *g) { delete g; }
 
 int GuidePrepareWave(GuideState &g, WaveBuffers &W, WaveQueues &Q, uint32_t cap_q, uint32_t levels, cudaStream_t st) {
     if (W.guide_lobes_cap < cap_q) {
-        if (W.guide_lobes) cudaFree(W.guide_lobes);
+        PoolFree(W.guide_lobes, st);
         W.guide_lobes = nullptr;
         W.guide_lobes_cap = 0;
-        if (cudaMalloc((void **)&W.guide_lobes, (size_t)cap_q * sizeof(GuideLobes)) != cudaSuccess)
+        if (PoolAlloc((void **)&W.guide_lobes, (size_t)cap_q * sizeof(GuideLobes), st) != cudaSuccess)
             return SetError(AZ_ERR_OUT_OF_MEMORY, "path guide proposals");
         W.guide_lobes_cap = cap_q;
     }
@@ -1523,10 +1524,10 @@ int GuidePrepareWave(GuideState &g, WaveBuffers &W, WaveQueues &Q, uint32_t cap_
     if (levels == 0) return AZ_OK;   // not training: no records
     const size_t need = (size_t)levels * g.n_rec;
     if (W.guide_rec_cap < need) {
-        if (W.guide_rec) cudaFree(W.guide_rec);
+        PoolFree(W.guide_rec, st);
         W.guide_rec = nullptr;
         W.guide_rec_cap = 0;
-        if (cudaMalloc((void **)&W.guide_rec, need * sizeof(GuideRecord)) != cudaSuccess)
+        if (PoolAlloc((void **)&W.guide_rec, need * sizeof(GuideRecord), st) != cudaSuccess)
             return SetError(AZ_ERR_OUT_OF_MEMORY, "path guide records");
         W.guide_rec_cap = need;
     }

@@ -48,6 +48,7 @@ struct GpuScene {
     uint32_t bvh_builder = AZ_BVH_PLOC;   // binary hierarchy under the wide collapse
     bool from_soup = false;      // meshes came from az_gpu_scene_create_from_meshes
     size_t device_bytes = 0;
+    cudaStream_t build_stream = nullptr;   // orders the allocations of the build
     WaveBuffers waves;           // reused across render calls on this scene
     uint32_t variant = 7;        // traversal launch configuration, 0-based (ChooseDefaultVariants; az_gpu_autotune
                                  // picks per scene)

@@ -26,6 +26,7 @@
 #include <cstring>
 
 #include "az_internal.h"
+#include "az_pool.h"
 
 namespace az {
 namespace {
@@ -231,22 +232,13 @@ __global__ void k_ingest_copy(const IngestCopy *copies, const uint32_t *start, u
     attrs[C.dst + k] = a;
 }
 
-template <typename T>
-struct Dev {
-    T *p = nullptr;
-    ~Dev() {
-        if (p) cudaFree(p);
-    }
-    cudaError_t alloc(size_t n) { return cudaMalloc((void **)&p, (n ? n : 1) * sizeof(T)); }
-};
-
 }  // namespace
 
 struct SoupWork {
     uint32_t nv = 0, nf = 0, nuv = 0, nm = 0;
-    Dev<float> v, uv, fn_raw, fn_unit, half_area, vn, area;
-    Dev<uint32_t> faces;
-    Dev<MeshRange> ranges;
+    PoolBuf<float> v, uv, fn_raw, fn_unit, half_area, vn, area;
+    PoolBuf<uint32_t> faces;
+    PoolBuf<MeshRange> ranges;
 };
 
 void FreeSoupWork(SoupWork *w) { delete w; }
@@ -278,23 +270,23 @@ int IngestSoup(const az_mesh_soup *soup, cudaStream_t st, SoupWork **out) {
     W->nuv = soup->uv_count;
     W->nm = soup->mesh_count;
     const uint32_t nv = W->nv, nf = W->nf, n_inc = 3 * nf;
-    Dev<uint32_t> key, val, skey, sval, vstart, vend, err;
-    AZ_CUDA_TRY(W->v.alloc((size_t)3 * nv));
-    AZ_CUDA_TRY(W->uv.alloc((size_t)2 * W->nuv));
-    AZ_CUDA_TRY(W->faces.alloc((size_t)3 * nf));
-    AZ_CUDA_TRY(W->fn_raw.alloc((size_t)3 * nf));
-    AZ_CUDA_TRY(W->fn_unit.alloc((size_t)3 * nf));
-    AZ_CUDA_TRY(W->half_area.alloc(nf));
-    AZ_CUDA_TRY(W->vn.alloc((size_t)3 * nv));
-    AZ_CUDA_TRY(W->area.alloc(W->nm));
-    AZ_CUDA_TRY(W->ranges.alloc(W->nm));
-    AZ_CUDA_TRY(key.alloc(n_inc));
-    AZ_CUDA_TRY(val.alloc(n_inc));
-    AZ_CUDA_TRY(skey.alloc(n_inc));
-    AZ_CUDA_TRY(sval.alloc(n_inc));
-    AZ_CUDA_TRY(vstart.alloc(nv));
-    AZ_CUDA_TRY(vend.alloc(nv));
-    AZ_CUDA_TRY(err.alloc(1));
+    PoolBuf<uint32_t> key, val, skey, sval, vstart, vend, err;
+    AZ_CUDA_TRY(W->v.alloc((size_t)3 * nv, st));
+    AZ_CUDA_TRY(W->uv.alloc((size_t)2 * W->nuv, st));
+    AZ_CUDA_TRY(W->faces.alloc((size_t)3 * nf, st));
+    AZ_CUDA_TRY(W->fn_raw.alloc((size_t)3 * nf, st));
+    AZ_CUDA_TRY(W->fn_unit.alloc((size_t)3 * nf, st));
+    AZ_CUDA_TRY(W->half_area.alloc(nf, st));
+    AZ_CUDA_TRY(W->vn.alloc((size_t)3 * nv, st));
+    AZ_CUDA_TRY(W->area.alloc(W->nm, st));
+    AZ_CUDA_TRY(W->ranges.alloc(W->nm, st));
+    AZ_CUDA_TRY(key.alloc(n_inc, st));
+    AZ_CUDA_TRY(val.alloc(n_inc, st));
+    AZ_CUDA_TRY(skey.alloc(n_inc, st));
+    AZ_CUDA_TRY(sval.alloc(n_inc, st));
+    AZ_CUDA_TRY(vstart.alloc(nv, st));
+    AZ_CUDA_TRY(vend.alloc(nv, st));
+    AZ_CUDA_TRY(err.alloc(1, st));
     if (nv) AZ_CUDA_TRY(cudaMemcpyAsync(W->v.p, soup->vertices, (size_t)nv * 12, cudaMemcpyHostToDevice, st));
     if (W->nuv) AZ_CUDA_TRY(cudaMemcpyAsync(W->uv.p, soup->uvs, (size_t)W->nuv * 8, cudaMemcpyHostToDevice, st));
     if (nf) AZ_CUDA_TRY(cudaMemcpyAsync(W->faces.p, soup->faces, (size_t)nf * 12, cudaMemcpyHostToDevice, st));
@@ -318,8 +310,8 @@ int IngestSoup(const az_mesh_soup *soup, cudaStream_t st, SoupWork **out) {
         size_t temp_bytes = 0;
         AZ_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, key.p, skey.p, val.p, sval.p, (int)n_inc, 0,
                                                     end_bit, st));
-        Dev<unsigned char> temp;
-        AZ_CUDA_TRY(temp.alloc(temp_bytes));
+        PoolBuf<unsigned char> temp;
+        AZ_CUDA_TRY(temp.alloc(temp_bytes, st));
         AZ_CUDA_TRY(cub::DeviceRadixSort::SortPairs(temp.p, temp_bytes, key.p, skey.p, val.p, sval.p, (int)n_inc, 0,
                                                     end_bit, st));
         k_ingest_segments<<<(n_inc + B - 1) / B, B, 0, st>>>(skey.p, n_inc, vstart.p, vend.p);
@@ -350,10 +342,10 @@ int SoupRecords(const SoupWork &w, az_triangle *tris, az_face_attr *attrs, az_ve
     if (vertex_normals && w.nv)
         AZ_CUDA_TRY(cudaMemcpy(vertex_normals, w.vn.p, (size_t)w.nv * 12, cudaMemcpyDeviceToHost));
     if ((!tris && !attrs) || w.nf == 0) return AZ_OK;
-    Dev<az_triangle> dt;
-    Dev<az_face_attr> da;
-    if (tris) AZ_CUDA_TRY(dt.alloc(w.nf));
-    if (attrs) AZ_CUDA_TRY(da.alloc(w.nf));
+    PoolBuf<az_triangle> dt;
+    PoolBuf<az_face_attr> da;
+    if (tris) AZ_CUDA_TRY(dt.alloc(w.nf, st));
+    if (attrs) AZ_CUDA_TRY(da.alloc(w.nf, st));
     k_ingest_emit_records<<<(w.nf + 255) / 256, 256, 0, st>>>(w.v.p, w.faces.p, 0, w.nf, w.fn_unit.p, w.vn.p, w.uv.p,
                                                              w.nuv, w.ranges.p, w.nm, dt.p, da.p);
     AZ_CUDA_TRY(cudaGetLastError());
@@ -396,8 +388,8 @@ __global__ void k_ingest_boxes(const float *v, const uint32_t *faces, const Mesh
 int SoupBoxes(const SoupWork &w, std::vector<float> &boxes, cudaStream_t st) {
     boxes.assign(6 * (size_t)w.nm, 0.0f);
     if (w.nm == 0) return AZ_OK;
-    Dev<float> d;
-    AZ_CUDA_TRY(d.alloc(boxes.size()));
+    PoolBuf<float> d;
+    AZ_CUDA_TRY(d.alloc(boxes.size(), st));
     k_ingest_boxes<<<w.nm, 256, 0, st>>>(w.v.p, w.faces.p, w.ranges.p, d.p);
     AZ_CUDA_TRY(cudaGetLastError());
     AZ_CUDA_TRY(cudaMemcpyAsync(boxes.data(), d.p, boxes.size() * sizeof(float), cudaMemcpyDeviceToHost, st));
@@ -408,8 +400,8 @@ int SoupBoxes(const SoupWork &w, std::vector<float> &boxes, cudaStream_t st) {
 int SoupTriangles(const SoupWork &w, uint32_t face_base, uint32_t count, az_triangle *tris, cudaStream_t st) {
     if (count == 0) return AZ_OK;
     if ((uint64_t)face_base + count > w.nf) return SetError(AZ_ERR_INVALID_SCENE, "face range outside the soup");
-    Dev<az_triangle> dt;
-    AZ_CUDA_TRY(dt.alloc(count));
+    PoolBuf<az_triangle> dt;
+    AZ_CUDA_TRY(dt.alloc(count, st));
     k_ingest_emit_records<<<(count + 255) / 256, 256, 0, st>>>(w.v.p, w.faces.p, face_base, count, w.fn_unit.p,
                                                               w.vn.p, w.uv.p, w.nuv, w.ranges.p, w.nm, dt.p, nullptr);
     AZ_CUDA_TRY(cudaGetLastError());
@@ -421,8 +413,8 @@ int SoupTriangles(const SoupWork &w, uint32_t face_base, uint32_t count, az_tria
 int SoupEmitScene(const SoupWork &w, const std::vector<IngestMesh> &meshes, azd::DevTriVerts *d_tris,
                   azd::DevTriAttr *d_attr, cudaStream_t st) {
     if (w.nf == 0 || w.nm == 0) return AZ_OK;
-    Dev<IngestMesh> dm;
-    AZ_CUDA_TRY(dm.alloc(meshes.size()));
+    PoolBuf<IngestMesh> dm;
+    AZ_CUDA_TRY(dm.alloc(meshes.size(), st));
     AZ_CUDA_TRY(cudaMemcpyAsync(dm.p, meshes.data(), meshes.size() * sizeof(IngestMesh), cudaMemcpyHostToDevice, st));
     k_ingest_emit_scene<<<(w.nf + 255) / 256, 256, 0, st>>>(w.v.p, w.faces.p, w.nf, w.fn_unit.p, w.vn.p, w.uv.p, w.nuv,
                                                            w.ranges.p, w.nm, dm.p, d_tris, d_attr);
@@ -442,10 +434,10 @@ int SoupCopyPlacements(const std::vector<IngestCopy> &copies, azd::DevTriVerts *
     }
     if (total >= (1ull << 31)) return SetError(AZ_ERR_UNSUPPORTED, "more than 2^31 instanced primitives");
     if (total == 0) return AZ_OK;
-    Dev<IngestCopy> dc;
-    Dev<uint32_t> ds;
-    AZ_CUDA_TRY(dc.alloc(copies.size()));
-    AZ_CUDA_TRY(ds.alloc(copies.size()));
+    PoolBuf<IngestCopy> dc;
+    PoolBuf<uint32_t> ds;
+    AZ_CUDA_TRY(dc.alloc(copies.size(), st));
+    AZ_CUDA_TRY(ds.alloc(copies.size(), st));
     AZ_CUDA_TRY(cudaMemcpyAsync(dc.p, copies.data(), copies.size() * sizeof(IngestCopy), cudaMemcpyHostToDevice, st));
     AZ_CUDA_TRY(cudaMemcpyAsync(ds.p, start.data(), start.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
     k_ingest_copy<<<(uint32_t)((total + 255) / 256), 256, 0, st>>>(dc.p, ds.p, (uint32_t)copies.size(),

@@ -1,0 +1,105 @@
+#include "az_pool.h"
+
+#include <mutex>
+#include <vector>
+
+namespace az {
+namespace {
+
+constexpr int kMaxDevices = 64;
+
+struct DevicePools {
+    std::mutex mu;
+    cudaMemPool_t pool[kMaxDevices] = {};
+    std::vector<cudaStream_t> streams[kMaxDevices];
+};
+
+// Never destroyed: the driver may be gone when static destructors run.
+DevicePools &Pools() {
+    static DevicePools *p = new DevicePools();
+    return *p;
+}
+
+cudaError_t PoolOf(int dev, cudaMemPool_t *out) {
+    if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
+    DevicePools &P = Pools();
+    std::lock_guard<std::mutex> lock(P.mu);
+    if (!P.pool[dev]) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool = nullptr;
+        cudaError_t e = cudaMemPoolCreate(&pool, &props);
+        if (e != cudaSuccess) return e;
+        unsigned long long kept = kPoolKept;
+        e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &kept);
+        if (e != cudaSuccess) {
+            cudaMemPoolDestroy(pool);
+            return e;
+        }
+        P.pool[dev] = pool;
+    }
+    *out = P.pool[dev];
+    return cudaSuccess;
+}
+
+}  // namespace
+
+cudaError_t PoolAlloc(void **p, size_t bytes, cudaStream_t st) {
+    *p = nullptr;
+    int dev = 0;
+    cudaMemPool_t pool = nullptr;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = PoolOf(dev, &pool);
+    if (e != cudaSuccess) return e;
+    e = cudaMallocFromPoolAsync(p, bytes, pool, st);
+    if (e == cudaErrorMemoryAllocation) {
+        // what the pool keeps may be in the way of a large buffer
+        cudaGetLastError();
+        cudaStreamSynchronize(st);
+        cudaMemPoolTrimTo(pool, 0);
+        e = cudaMallocFromPoolAsync(p, bytes, pool, st);
+    }
+    if (e != cudaSuccess) {
+        *p = nullptr;
+        cudaGetLastError();
+    }
+    return e;
+}
+
+void PoolFree(void *p, cudaStream_t st) {
+    if (p) cudaFreeAsync(p, st);
+}
+
+cudaError_t AcquireStream(cudaStream_t *st) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev >= 0 && dev < kMaxDevices) {
+        DevicePools &P = Pools();
+        std::lock_guard<std::mutex> lock(P.mu);
+        if (!P.streams[dev].empty()) {
+            *st = P.streams[dev].back();
+            P.streams[dev].pop_back();
+            return cudaSuccess;
+        }
+    }
+    return cudaStreamCreate(st);
+}
+
+void ReleaseStream(cudaStream_t st) {
+    cudaStreamSynchronize(st);
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices) {
+        DevicePools &P = Pools();
+        std::lock_guard<std::mutex> lock(P.mu);
+        if (P.streams[dev].size() < kStreamsKept) {
+            P.streams[dev].push_back(st);
+            return;
+        }
+    }
+    cudaStreamDestroy(st);
+}
+
+}  // namespace az

@@ -1,0 +1,46 @@
+// Device scratch and private streams that outlive a call.
+//
+// cudaMalloc and cudaFree wait for the device and take from tens of
+// microseconds to several milliseconds each (a build allocates about a hundred
+// buffers); a stream-ordered pool hands the same memory to the next call.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <cstddef>
+
+namespace az {
+
+// Memory of the current device's pool, usable by work on `st` from here on
+// (and by other streams once they are ordered after `st`).  The pool keeps at
+// most kPoolKept unused bytes across synchronisations; the rest goes back to
+// the driver.  Safe with several threads and streams.
+constexpr size_t kPoolKept = (size_t)512 << 20;
+cudaError_t PoolAlloc(void **p, size_t bytes, cudaStream_t st);
+// Gives memory back once the work queued on `st` so far has finished.
+void PoolFree(void *p, cudaStream_t st);
+
+// An array of the pool that lives as long as this object, used on one stream.
+template <typename T>
+struct PoolBuf {
+    T *p = nullptr;
+    cudaStream_t st = nullptr;
+    PoolBuf() = default;
+    PoolBuf(const PoolBuf &) = delete;
+    PoolBuf &operator=(const PoolBuf &) = delete;
+    ~PoolBuf() {
+        if (p) PoolFree(p, st);
+    }
+    cudaError_t alloc(size_t n, cudaStream_t s) {
+        st = s;
+        return PoolAlloc((void **)&p, (n ? n : 1) * sizeof(T) + 16, s);
+    }
+};
+
+// A blocking stream of the current device for one call (ordered after earlier
+// work on the legacy default stream); at most kStreamsKept idle ones are kept
+// per device.  ReleaseStream waits for the stream's work.
+constexpr size_t kStreamsKept = 8;
+cudaError_t AcquireStream(cudaStream_t *st);
+void ReleaseStream(cudaStream_t st);
+
+}  // namespace az

@@ -31,6 +31,7 @@
 
 #include "az_internal.h"
 #include "az_phase.cuh"
+#include "az_pool.h"
 #include "az_render.h"
 #include "az_shade.cuh"
 #include "az_wave.cuh"
@@ -586,13 +587,13 @@ int SetupCamera(const az_camera *c, az_scissor sc, int32_t filter, uint32_t cull
 
 WaveBuffers::~WaveBuffers() {
     DropGraph();
-    for (void *p : ptrs)
-        if (p) cudaFree(p);
+    // every render waits for its waves, so nothing uses the buffers any more
+    for (void *p : ptrs) PoolFree(p, nullptr);
     if (wave_host) cudaFreeHost(wave_host);
-    if (guide_lobes) cudaFree(guide_lobes);
-    if (guide_rec) cudaFree(guide_rec);
+    PoolFree(guide_lobes, nullptr);
+    PoolFree(guide_rec, nullptr);
     for (void *p : {(void *)okey[0], (void *)okey[1], (void *)oval, (void *)oidx_e, (void *)oidx_s, otemp})
-        if (p) cudaFree(p);
+        PoolFree(p, nullptr);
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
     if (side) cudaStreamDestroy(side);
@@ -618,27 +619,22 @@ int WaveBuffers::EnsureSide() {
     return AZ_OK;
 }
 
-int WaveBuffers::EnsureOrder(uint32_t cap) {
+int WaveBuffers::EnsureOrder(uint32_t cap, cudaStream_t st) {
     if (cap <= ocap && otemp) return AZ_OK;
     DropGraph();   // it refers to the buffers replaced below
     for (uint32_t **p : {&okey[0], &okey[1], &oval, &oidx_e, &oidx_s}) {
-        if (*p) cudaFree(*p);
+        PoolFree(*p, st);
         *p = nullptr;
     }
-    if (otemp) cudaFree(otemp);
+    PoolFree(otemp, st);
     otemp = nullptr;
     ocap = 0;
     for (uint32_t **p : {&okey[0], &okey[1], &oval, &oidx_e, &oidx_s})
-        if (cudaMalloc((void **)p, (size_t)cap * sizeof(uint32_t)) != cudaSuccess) {
-            *p = nullptr;
+        if (PoolAlloc((void **)p, (size_t)cap * sizeof(uint32_t), st) != cudaSuccess)
             return SetError(AZ_ERR_OUT_OF_MEMORY, "queue ordering buffers");
-        }
     size_t bytes = 0;
     AZ_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, bytes, okey[0], okey[1], oval, oidx_e, (int)cap, 0, 16));
-    if (cudaMalloc(&otemp, bytes) != cudaSuccess) {
-        otemp = nullptr;
-        return SetError(AZ_ERR_OUT_OF_MEMORY, "queue ordering scratch");
-    }
+    if (PoolAlloc(&otemp, bytes, st) != cudaSuccess) return SetError(AZ_ERR_OUT_OF_MEMORY, "queue ordering scratch");
     otemp_bytes = bytes;
     ocap = cap;
     return AZ_OK;
@@ -650,16 +646,15 @@ void WaveBuffers::DropGraph() {
     graph_key.clear();
 }
 
-int WaveBuffers::Ensure(uint32_t chunk, uint32_t cap_q, uint32_t cap_s) {
+int WaveBuffers::Ensure(uint32_t chunk, uint32_t cap_q, uint32_t cap_s, cudaStream_t st) {
     if (chunk <= this->chunk && cap_q <= q.cap_q && cap_s <= q.cap_s && !ptrs.empty()) return AZ_OK;
     DropGraph();   // it refers to the buffers freed below
-    for (void *p : ptrs)
-        if (p) cudaFree(p);
+    for (void *p : ptrs) PoolFree(p, st);
     ptrs.clear();
     memset(&q, 0, sizeof(q));
     auto alloc = [&](size_t bytes) -> void * {
         void *p = nullptr;
-        if (cudaMalloc(&p, bytes) != cudaSuccess) return nullptr;
+        if (PoolAlloc(&p, bytes, st) != cudaSuccess) return nullptr;
         ptrs.push_back(p);
         return p;
     };
@@ -952,8 +947,9 @@ static uint32_t QueueOrder(const GpuScene &G, const az_render_opts *opts) {
 // have ended, full (C1: 427 ms per frame at 2^22, 393 at 2^24, 383 at 2^26).
 // The queues `W` already holds count as free, so that repeated renders of a
 // scene keep their wave size.
-static uint32_t DefaultWave(uint32_t per_node_shadow, const WaveBuffers &W) {
+static uint32_t DefaultWave(uint32_t per_node_shadow, const WaveBuffers &W, uint64_t total) {
     uint64_t n = 1u << 22;
+    if (total <= n) return (uint32_t)n;   // one wave of the smallest size holds the render
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
         cudaGetLastError();
@@ -1001,7 +997,7 @@ int Render(GpuScene &G, az_pixel *film, const az_camera *camera, const az_epsilo
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, G.device);
     uint32_t per_node_shadow = G.dev.light_count + (G.dev.use_env_map ? 1u : 0u);
     WaveBuffers &W = wave_buffers ? *wave_buffers : G.waves;
-    uint32_t chunk = opts && opts->chunk_samples ? opts->chunk_samples : DefaultWave(per_node_shadow, W);
+    uint32_t chunk = opts && opts->chunk_samples ? opts->chunk_samples : DefaultWave(per_node_shadow, W, total);
     // a training render updates the guide after every wave: smaller waves, more updates
     if (guide && train && !(opts && opts->chunk_samples)) chunk = 1u << 20;
     // the visit counters are 32-bit per wave: counting renders keep 2^22-sample waves
@@ -1030,9 +1026,9 @@ int Render(GpuScene &G, az_pixel *film, const az_camera *camera, const az_epsilo
         uint32_t cap_q = std::max<uint32_t>(n + n / 2, 1024);
         uint32_t cap_s = std::max<uint32_t>((uint32_t)std::min<uint64_t>((uint64_t)cap_q * std::max(per_node_shadow, 1u),
                                                                          (uint64_t)n * 4), 1024);
-        rc = W.Ensure(n, cap_q, cap_s);
+        rc = W.Ensure(n, cap_q, cap_s, st);
         if (rc != AZ_OK) return rc;
-        if (cam.order && (rc = W.EnsureOrder(std::max(W.q.cap_q, W.q.cap_s))) != AZ_OK) return rc;
+        if (cam.order && (rc = W.EnsureOrder(std::max(W.q.cap_q, W.q.cap_s), st)) != AZ_OK) return rc;
         if (!cam.serial_levels && (rc = W.EnsureSide()) != AZ_OK) return rc;
         if (use_graph) {
             rc = ReplayWave(G, cam, W, pos, n, chunk, film, st, sms, counters);
@@ -1166,29 +1162,29 @@ int RenderTiles(GpuScene &G, std::vector<TileJob> &jobs, const az_render_opts *o
     }
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, G.device);
-    uint32_t chunk = opts && opts->chunk_samples ? opts->chunk_samples : DefaultWave(per_node_shadow, G.waves);
+    uint32_t chunk = opts && opts->chunk_samples ? opts->chunk_samples : DefaultWave(per_node_shadow, G.waves, total);
     chunk = std::max<uint32_t>(chunk, kTile);
     WaveBuffers &W = G.waves;
     // device tables: cameras, films, this wave's tiles, the work-queue counter, slot -> (job, sample)
-    struct DevBuf {
-        void *p = nullptr;
-        ~DevBuf() {
-            if (p) cudaFree(p);
-        }
-    } d_cams, d_films, d_tiles, d_next, d_slots, d_scenes;
+    PoolBuf<CameraParams> d_cams;
+    PoolBuf<az_pixel *> d_films;
+    PoolBuf<Tile> d_tiles;
+    PoolBuf<uint32_t> d_next;
+    PoolBuf<uint2> d_slots;
+    PoolBuf<DevScene> d_scenes;
     std::vector<az_pixel *> films(nj);
     for (uint32_t j = 0; j < nj; j++) films[j] = jobs[j].film;
-    AZ_CUDA_TRY(cudaMalloc(&d_cams.p, nj * sizeof(CameraParams)));
-    AZ_CUDA_TRY(cudaMalloc(&d_films.p, nj * sizeof(az_pixel *)));
-    AZ_CUDA_TRY(cudaMalloc(&d_tiles.p, (chunk / kTile + 2 + nj) * sizeof(Tile)));
-    AZ_CUDA_TRY(cudaMalloc(&d_next.p, sizeof(uint32_t)));
-    AZ_CUDA_TRY(cudaMalloc(&d_slots.p, (size_t)chunk * sizeof(uint2)));
+    AZ_CUDA_TRY(d_cams.alloc(nj, st));
+    AZ_CUDA_TRY(d_films.alloc(nj, st));
+    AZ_CUDA_TRY(d_tiles.alloc(chunk / kTile + 2 + nj, st));
+    AZ_CUDA_TRY(d_next.alloc(1, st));
+    AZ_CUDA_TRY(d_slots.alloc(chunk, st));
     AZ_CUDA_TRY(cudaMemcpyAsync(d_cams.p, cams.data(), nj * sizeof(CameraParams), cudaMemcpyHostToDevice, st));
     AZ_CUDA_TRY(cudaMemcpyAsync(d_films.p, films.data(), nj * sizeof(az_pixel *), cudaMemcpyHostToDevice, st));
     std::vector<DevScene> scene_recs;
     if (multi) {
         for (GpuScene *sg : scenes) scene_recs.push_back(sg->dev);
-        AZ_CUDA_TRY(cudaMalloc(&d_scenes.p, scene_recs.size() * sizeof(DevScene)));
+        AZ_CUDA_TRY(d_scenes.alloc(scene_recs.size(), st));
         AZ_CUDA_TRY(cudaMemcpyAsync(d_scenes.p, scene_recs.data(), scene_recs.size() * sizeof(DevScene),
                                     cudaMemcpyHostToDevice, st));
     }
@@ -1219,14 +1215,13 @@ int RenderTiles(GpuScene &G, std::vector<TileJob> &jobs, const az_render_opts *o
         const uint32_t cap_q = std::max<uint32_t>(n + n / 2, 1024);
         const uint32_t cap_s = std::max<uint32_t>(
             (uint32_t)std::min<uint64_t>((uint64_t)cap_q * std::max(per_node_shadow, 1u), (uint64_t)n * 4), 1024);
-        int rc = W.Ensure(n, cap_q, cap_s);
+        int rc = W.Ensure(n, cap_q, cap_s, st);
         if (rc != AZ_OK) return rc;
-        if (cams[0].order && (rc = W.EnsureOrder(std::max(W.q.cap_q, W.q.cap_s))) != AZ_OK) return rc;
+        if (cams[0].order && (rc = W.EnsureOrder(std::max(W.q.cap_q, W.q.cap_s), st)) != AZ_OK) return rc;
         if (!cams[0].serial_levels && (rc = W.EnsureSide()) != AZ_OK) return rc;
         AZ_CUDA_TRY(cudaMemcpyAsync(d_tiles.p, tiles.data() + ti, ntiles * sizeof(Tile), cudaMemcpyHostToDevice, st));
-        TileWave tw{(const Tile *)d_tiles.p, ntiles, (uint32_t *)d_next.p, (uint2 *)d_slots.p,
-                    (const CameraParams *)d_cams.p, (az_pixel *const *)d_films.p,
-                    multi ? (const DevScene *)d_scenes.p : nullptr, multi ? &wave_dev : nullptr};
+        TileWave tw{d_tiles.p, ntiles, d_next.p, d_slots.p, d_cams.p, d_films.p,
+                    multi ? d_scenes.p : nullptr, multi ? &wave_dev : nullptr};
         rc = RenderWave(G, cams[0], W, 0, n, nullptr, st, sms, counters, nullptr, nullptr, false, false, &tw);
         if (rc != AZ_OK) return rc;
         AZ_CUDA_TRY(cudaMemcpyAsync(host_counts.data(), W.q.counts, AZ_COUNT_TOTAL * sizeof(uint32_t),
@@ -1398,10 +1393,9 @@ __global__ void k_closest(DevScene S, const az_ray3 *rays, uint32_t n, uint32_t 
 int ClosestHit(GpuScene &G, const az_ray3 *rays, uint32_t n, int32_t cull, float eps, uint32_t *out_hit,
                uint32_t *out_uid, uint32_t *out_face, float *out_t, cudaStream_t st, bool watertight) {
     if (n == 0) return AZ_OK;
-    void *buf = nullptr;
-    size_t bytes = (size_t)n * (sizeof(az_ray3) + 3 * sizeof(uint32_t) + sizeof(float)) + 64;
-    AZ_CUDA_TRY(cudaMalloc(&buf, bytes));
-    char *p = (char *)buf;
+    PoolBuf<char> buf;
+    AZ_CUDA_TRY(buf.alloc((size_t)n * (sizeof(az_ray3) + 3 * sizeof(uint32_t) + sizeof(float)) + 64, st));
+    char *p = buf.p;
     az_ray3 *d_rays = (az_ray3 *)p;
     p += ((size_t)n * sizeof(az_ray3) + 15) & ~(size_t)15;
     uint32_t *d_hit = (uint32_t *)p;
@@ -1425,7 +1419,6 @@ int ClosestHit(GpuScene &G, const az_ray3 *rays, uint32_t n, int32_t cull, float
     if (e == cudaSuccess) e = cudaMemcpyAsync(out_t, d_t, n * 4, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) rc = CudaError(e, "closest-hit query");
-    cudaFree(buf);
     return rc;
 }
 

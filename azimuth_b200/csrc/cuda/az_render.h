@@ -122,9 +122,9 @@ struct WaveBuffers {
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     ~WaveBuffers();
     int EnsureSide();
-    int EnsureOrder(uint32_t cap);
+    int EnsureOrder(uint32_t cap, cudaStream_t st);
     void DropGraph();
-    int Ensure(uint32_t chunk, uint32_t cap_q, uint32_t cap_s);
+    int Ensure(uint32_t chunk, uint32_t cap_q, uint32_t cap_s, cudaStream_t st);
 };
 
 struct RenderCounters {

@@ -18,20 +18,21 @@
 #include <string>
 
 #include "az_internal.h"
+#include "az_pool.h"
 #include "az_scene_build.h"
 
 namespace az {
 
 GpuScene::~GpuScene() {
-    for (auto &b : bufs)
-        if (b.ptr) cudaFree(b.ptr);
-    if (host_film_dev) cudaFree(host_film_dev);
+    cudaDeviceSynchronize();   // its buffers may still be in use, on any stream
+    for (auto &b : bufs) PoolFree(b.ptr, nullptr);
+    PoolFree(host_film_dev, nullptr);
 }
 
 void *GpuScene::Alloc(size_t bytes) {
     void *p = nullptr;
     if (bytes == 0) bytes = 16;
-    if (cudaMalloc(&p, bytes) != cudaSuccess) return nullptr;
+    if (PoolAlloc(&p, bytes, build_stream) != cudaSuccess) return nullptr;
     bufs.push_back(DevBuf{p, bytes});
     device_bytes += bytes;
     return p;
@@ -363,16 +364,6 @@ T *Upload(GpuScene &G, const std::vector<T> &v, cudaStream_t st, int &rc) {
     return p;
 }
 
-// A device buffer that lives only while the scene is built.
-template <typename T>
-struct TempBuf {
-    T *p = nullptr;
-    ~TempBuf() {
-        if (p) cudaFree(p);
-    }
-    bool alloc(size_t n) { return cudaMalloc((void **)&p, (n ? n : 1) * sizeof(T)) != cudaSuccess; }   // true on failure
-};
-
 // The primitives in wide-leaf order: the exact vertices, and the operands of
 // azimuth's Cramer test -- P0, E1 = P0 - P1 and E2 = P0 - P2 in float, the
 // A..H of src/azimuth_main.cpp:154-164 (a float subtraction rounds the same
@@ -422,6 +413,7 @@ int BuildGpuScene(const az_scene *scene, const az_render_opts *opts, cudaStream_
     const auto t_start = std::chrono::steady_clock::now();
     std::unique_ptr<GpuScene> G(new GpuScene());
     G->device = opts ? opts->device : 0;
+    G->build_stream = st;
     const uint32_t width = opts && opts->bvh_width ? opts->bvh_width : 8u;
     if (width != 2 && width != 4 && width != 8) return SetError(AZ_ERR_INVALID_ARGUMENT, "bvh_width must be 0, 2, 4 or 8");
     G->bvh_width = width;
@@ -687,21 +679,21 @@ int BuildGpuScene(const az_scene *scene, const az_render_opts *opts, cudaStream_
     // Build-only buffers are freed when the build ends; the scene keeps the
     // sorted primitives, the wide nodes and the top-level primitive list.
     const size_t nmax = std::max((size_t)total_tris, tlas.size()) + 1;
-    TempBuf<azd::DevTriVerts> d_tris_unsorted;
-    TempBuf<azd::DevTriAttr> d_attr_unsorted;
-    TempBuf<azd::BVHNode> d_nodes;
-    TempBuf<uint2> d_range;
-    TempBuf<float4> d_lo, d_hi;
-    TempBuf<uint32_t> d_perm, d_comp, d_tlas_unsorted;
-    TempBuf<azd::WideNode> d_wide_tmp;
+    PoolBuf<azd::DevTriVerts> d_tris_unsorted;
+    PoolBuf<azd::DevTriAttr> d_attr_unsorted;
+    PoolBuf<azd::BVHNode> d_nodes;
+    PoolBuf<uint2> d_range;
+    PoolBuf<float4> d_lo, d_hi;
+    PoolBuf<uint32_t> d_perm, d_comp, d_tlas_unsorted;
+    PoolBuf<azd::WideNode> d_wide_tmp;
     azd::DevTri *d_tris = (azd::DevTri *)G->Alloc(total_tris * sizeof(azd::DevTri));
     azd::DevTriVerts *d_verts = (azd::DevTriVerts *)G->Alloc(total_tris * sizeof(azd::DevTriVerts));
     azd::DevTriAttr *d_attr = (azd::DevTriAttr *)G->Alloc(total_tris * sizeof(azd::DevTriAttr));
     uint32_t *d_tlas = (uint32_t *)G->Alloc((tlas.size() + 1) * sizeof(uint32_t));
-    if (!d_tris || !d_verts || !d_attr || !d_tlas || d_tris_unsorted.alloc(total_tris) ||
-        d_attr_unsorted.alloc(total_tris) || d_nodes.alloc(node_total) || d_range.alloc(node_total) ||
-        d_lo.alloc(nmax) || d_hi.alloc(nmax) || d_perm.alloc(nmax) || d_comp.alloc(nmax) ||
-        d_tlas_unsorted.alloc(tlas.size() + 1) || d_wide_tmp.alloc(node_total))
+    if (!d_tris || !d_verts || !d_attr || !d_tlas || d_tris_unsorted.alloc(total_tris, st) ||
+        d_attr_unsorted.alloc(total_tris, st) || d_nodes.alloc(node_total, st) || d_range.alloc(node_total, st) ||
+        d_lo.alloc(nmax, st) || d_hi.alloc(nmax, st) || d_perm.alloc(nmax, st) || d_comp.alloc(nmax, st) ||
+        d_tlas_unsorted.alloc(tlas.size() + 1, st) || d_wide_tmp.alloc(node_total, st))
         return SetError(AZ_ERR_OUT_OF_MEMORY, "device allocation failed");
     const auto t_up0 = std::chrono::steady_clock::now();
     for (auto &g : F.groups) {

@@ -24,6 +24,7 @@
 #include <cstring>
 
 #include "az_internal.h"
+#include "az_pool.h"
 
 namespace az {
 namespace {
@@ -279,15 +280,6 @@ __global__ void k_perm_check(const uint32_t *perm, uint32_t n, uint32_t *seen, u
     if (v >= n || atomicAdd(&seen[v], 1u) != 0) atomicOr(err, 2u);
 }
 
-template <typename T>
-struct DevScratch {
-    T *p = nullptr;
-    ~DevScratch() {
-        if (p) cudaFree(p);
-    }
-    cudaError_t alloc(size_t n) { return cudaMalloc((void **)&p, (n ? n : 1) * sizeof(T)); }
-};
-
 }  // namespace
 
 int CollapseToWide(const azd::BVHNode *d_nodes, const uint2 *d_range, uint32_t bin_root, uint32_t n,
@@ -299,18 +291,18 @@ int CollapseToWide(const azd::BVHNode *d_nodes, const uint2 *d_range, uint32_t b
     if (n == 0) return SetError(AZ_ERR_INVALID_ARGUMENT, "empty hierarchy");
     // a wide node per binary node at most: every node is made from a distinct one
     const uint32_t max_items = n > 1 ? n - 1 : 1;
-    DevScratch<CItem> items_a, items_b;
-    DevScratch<unsigned long long> counts, incl, total;
-    DevScratch<uint32_t> flags;   // [0] error bits, [1..n] permutation check
-    DevScratch<unsigned char> temp;
-    AZ_CUDA_TRY(items_a.alloc(max_items));
-    AZ_CUDA_TRY(items_b.alloc(max_items));
-    AZ_CUDA_TRY(counts.alloc(max_items));
-    AZ_CUDA_TRY(incl.alloc(max_items));
-    AZ_CUDA_TRY(flags.alloc((size_t)n + 1));
+    PoolBuf<CItem> items_a, items_b;
+    PoolBuf<unsigned long long> counts, incl, total;
+    PoolBuf<uint32_t> flags;   // [0] error bits, [1..n] permutation check
+    PoolBuf<unsigned char> temp;
+    AZ_CUDA_TRY(items_a.alloc(max_items, st));
+    AZ_CUDA_TRY(items_b.alloc(max_items, st));
+    AZ_CUDA_TRY(counts.alloc(max_items, st));
+    AZ_CUDA_TRY(incl.alloc(max_items, st));
+    AZ_CUDA_TRY(flags.alloc((size_t)n + 1, st));
     size_t temp_bytes = 0;
     AZ_CUDA_TRY(cub::DeviceScan::InclusiveSum(nullptr, temp_bytes, counts.p, incl.p, (int)max_items, st));
-    AZ_CUDA_TRY(temp.alloc(temp_bytes));
+    AZ_CUDA_TRY(temp.alloc(temp_bytes, st));
     AZ_CUDA_TRY(cudaMemsetAsync(flags.p, 0, ((size_t)n + 1) * sizeof(uint32_t), st));
 
     CParams P;
