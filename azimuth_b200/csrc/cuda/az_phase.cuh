@@ -117,7 +117,10 @@ struct PhaseShared {
     uint32_t mem[LM_COUNT][BLOCK];
 };
 
-template <QueryKind KIND, bool WT, bool SPH, int BLOCK>
+// MULTI: lanes of a warp may trace different scenes; a lane keeps the two array
+// addresses it needs in every round instead of reading them from its scene's
+// record each time.
+template <QueryKind KIND, bool WT, bool SPH, int BLOCK, bool MULTI>
 struct PhaseTracer {
     PhaseShared<BLOCK> &sh;
     uint2 *deep;                 // stack entries beyond the shared ones: an array of the caller, so that this
@@ -133,6 +136,8 @@ struct PhaseTracer {
     bool in_blas, pg2;
     bool stopped, occluded;      // Q_ANY: stopped at a hit to be confirmed; something lies closer than tmax
     WtRay wt;
+    const WideNode *own_nodes;   // MULTI
+    const float4 *own_tris;
 
     __device__ __forceinline__ PhaseTracer(PhaseShared<BLOCK> &s, uint2 *lower) : sh(s), deep(lower) {}
     __device__ __forceinline__ uint32_t &mem(int k) { return sh.mem[k][threadIdx.x]; }
@@ -178,6 +183,10 @@ struct PhaseTracer {
             mem(LM_B) = 0u;
             mem(LM_C) = 0xFFFFFFFFu;
             mem(LM_D) = 0xFFFFFFFFu;
+        }
+        if (MULTI) {
+            own_nodes = S.wnodes;
+            own_tris = WT ? (const float4 *)S.tri_verts : (const float4 *)S.tris;
         }
         bl_t = FLT_MAX;
         pg_base = pg_lo = pg_hi = 0u;
@@ -296,7 +305,7 @@ struct PhaseTracer {
         const uint32_t key = 31u - __clz(ng_bits & 0xFFu);
         const uint32_t slot = key ^ perm, imask = ng_bits >> 8;
         const uint32_t n = ng_base + __popc(imask & ((1u << slot) - 1u));
-        const uint4 *np = reinterpret_cast<const uint4 *>(S.wnodes + n);
+        const uint4 *np = reinterpret_cast<const uint4 *>((MULTI ? own_nodes : S.wnodes) + n);
         const uint4 w0 = __ldg(np + 0), w1 = __ldg(np + 1), w2 = __ldg(np + 2), w3 = __ldg(np + 3),
                     w4 = __ldg(np + 4);
         ng_bits ^= 1u << key;
@@ -338,8 +347,8 @@ struct PhaseTracer {
         if (in_blas) {
             float t, bt, gm;
             bool hit;
-            if (WT) hit = tri_test_wt(load_tri_verts(S.tri_verts, pi), ray(), wt, cull, eps, bl_t, t);
-            else hit = tri_test(load_tri(S.tris, pi), ray(), cull, eps, bl_t, t, bt, gm);
+            if (WT) hit = tri_test_wt(load_tri_verts(MULTI ? (const DevTriVerts *)own_tris : S.tri_verts, pi), ray(), wt, cull, eps, bl_t, t);
+            else hit = tri_test(load_tri(MULTI ? (const DevTri *)own_tris : S.tris, pi), ray(), cull, eps, bl_t, t, bt, gm);
             if (!hit) return false;
             if (KIND == Q_ANY) {
                 // a primitive of the skipped entity is ignored; its owner is

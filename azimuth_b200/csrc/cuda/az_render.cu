@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(kTraceBlock, MINB ? MINB : 8)
     }
     __shared__ PhaseShared<kTraceBlock> shared;
     uint2 deep[AZD_WSTACK - kSharedStack];
-    PhaseTracer<Q_CLOSEST, WT, SPH, kTraceBlock> T(shared, deep);
+    PhaseTracer<Q_CLOSEST, WT, SPH, kTraceBlock, MULTI> T(shared, deep);
     const int buf = level & 1;
     uint32_t si = 0;   // MULTI: the entry's scene
     auto load = [&](uint32_t q) {
@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(kTraceBlock, MINB ? MINB : 8)
     }
     __shared__ PhaseShared<kTraceBlock> shared;
     uint2 deep[AZD_WSTACK - kSharedStack];
-    PhaseTracer<Q_ANY, WT, SPH, kTraceBlock> T(shared, deep);
+    PhaseTracer<Q_ANY, WT, SPH, kTraceBlock, MULTI> T(shared, deep);
     uint32_t si = 0;   // MULTI: the entry's scene
     auto load = [&](uint32_t q) {
         const float4 o = Q.so[q], d = Q.sd[q];
@@ -510,9 +510,11 @@ void LaunchTraversalVariant(uint32_t v, bool shadow, int sms, const DevScene &S,
         else if (cam.watertight) k_shadow_full<true><<<grid, 128, 0, st>>>(S, cam, Q, L);
         else k_shadow_full<false><<<grid, 128, 0, st>>>(S, cam, Q, L);
     }
-    // a tile wave of several scenes and the watertight test have one block count
+    // A tile wave of several scenes and the watertight test have one block count:
+    // their lanes keep more state (24 jobs of three scenes: 28.1 ms with 7 blocks,
+    // 29.2 with 8, whose kernels spill)
     if (Q.scenes && cam.watertight) LaunchTraversal<7, true, true>(shadow, sms, S, cam, Q, L, st);
-    else if (Q.scenes) LaunchTraversal<8, false, true>(shadow, sms, S, cam, Q, L, st);
+    else if (Q.scenes) LaunchTraversal<7, false, true>(shadow, sms, S, cam, Q, L, st);
     else if (cam.watertight) LaunchTraversal<7, true, false>(shadow, sms, S, cam, Q, L, st);
     else if (loop) LaunchTraversal<0, false, false>(shadow, sms, S, cam, Q, L, st);
     else if (kVariants[v].minb == 7) LaunchTraversal<7, false, false>(shadow, sms, S, cam, Q, L, st);
@@ -1151,11 +1153,16 @@ int RenderTiles(GpuScene &G, std::vector<TileJob> &jobs, const az_render_opts *o
     }
     if (total == 0) return AZ_OK;
     // every job's samples in runs of kTile consecutive sample indices (one
-    // sample number over a run of pixels: coherent camera rays), jobs in order
+    // sample number over a run of pixels: coherent camera rays), jobs of one
+    // scene after another: a warp's lanes then mostly read one scene
     constexpr uint32_t kTile = 4096;
     std::vector<Tile> tiles;
     std::vector<size_t> last_tile(nj, 0);
-    for (uint32_t j = 0; j < nj; j++) {
+    std::vector<uint32_t> by_scene(nj);
+    for (uint32_t j = 0; j < nj; j++) by_scene[j] = j;
+    std::stable_sort(by_scene.begin(), by_scene.end(),
+                     [&](uint32_t a, uint32_t b) { return scene_of[a] < scene_of[b]; });
+    for (uint32_t j : by_scene) {
         for (uint64_t first = 0; first < jobs[j].samples; first += kTile)
             tiles.push_back(Tile{j, (uint32_t)first, (uint32_t)std::min<uint64_t>(kTile, jobs[j].samples - first), 0u});
         last_tile[j] = tiles.size();   // one past the job's last tile
@@ -1163,7 +1170,7 @@ int RenderTiles(GpuScene &G, std::vector<TileJob> &jobs, const az_render_opts *o
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, G.device);
     uint32_t chunk = opts && opts->chunk_samples ? opts->chunk_samples : DefaultWave(per_node_shadow, G.waves, total);
-    chunk = std::max<uint32_t>(chunk, kTile);
+    chunk = std::max<uint32_t>((uint32_t)std::min<uint64_t>(chunk, total), kTile);
     WaveBuffers &W = G.waves;
     // device tables: cameras, films, this wave's tiles, the work-queue counter, slot -> (job, sample)
     PoolBuf<CameraParams> d_cams;
