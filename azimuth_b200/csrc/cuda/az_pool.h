@@ -14,7 +14,7 @@ namespace az {
 // (and by other streams once they are ordered after `st`).  The pool keeps at
 // most kPoolKept unused bytes across synchronisations; the rest goes back to
 // the driver.  Safe with several threads and streams.
-constexpr size_t kPoolKept = (size_t)512 << 20;
+constexpr size_t kPoolKept = (size_t)2 << 30;
 cudaError_t PoolAlloc(void **p, size_t bytes, cudaStream_t st);
 // Gives memory back once the work queued on `st` so far has finished.
 void PoolFree(void *p, cudaStream_t st);
