@@ -1,6 +1,7 @@
 #include "az_pool.h"
 
 #include <mutex>
+#include <unordered_set>
 #include <vector>
 
 namespace az {
@@ -12,6 +13,8 @@ struct DevicePools {
     std::mutex mu;
     cudaMemPool_t pool[kMaxDevices] = {};
     std::vector<cudaStream_t> streams[kMaxDevices];
+    cudaStream_t idle[kMaxDevices] = {};   // takes the frees of memory that no work uses any more
+    std::unordered_set<void *> direct;     // buffers of cudaMalloc
 };
 
 // Never destroyed: the driver may be gone when static destructors run.
@@ -51,6 +54,24 @@ cudaError_t PoolAlloc(void **p, size_t bytes, cudaStream_t st) {
     int dev = 0;
     cudaMemPool_t pool = nullptr;
     cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess && bytes > kPoolLargest) {
+        e = cudaMalloc(p, bytes);
+        if (e == cudaErrorMemoryAllocation) {
+            // what the pool keeps may be in the way
+            cudaGetLastError();
+            if (PoolOf(dev, &pool) == cudaSuccess && cudaStreamSynchronize(st) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
+            e = cudaMalloc(p, bytes);
+        }
+        if (e == cudaSuccess) {
+            DevicePools &P = Pools();
+            std::lock_guard<std::mutex> lock(P.mu);
+            P.direct.insert(*p);
+        } else {
+            *p = nullptr;
+            cudaGetLastError();
+        }
+        return e;
+    }
     if (e == cudaSuccess) e = PoolOf(dev, &pool);
     if (e != cudaSuccess) return e;
     e = cudaMallocFromPoolAsync(p, bytes, pool, st);
@@ -69,7 +90,26 @@ cudaError_t PoolAlloc(void **p, size_t bytes, cudaStream_t st) {
 }
 
 void PoolFree(void *p, cudaStream_t st) {
-    if (p) cudaFreeAsync(p, st);
+    if (!p) return;
+    DevicePools &P = Pools();
+    {
+        std::lock_guard<std::mutex> lock(P.mu);
+        if (P.direct.erase(p) == 0) {
+            // Not on the legacy default stream: a free queued there would break a
+            // capture that another thread has open on a stream of its own.
+            int dev = 0;
+            if (!st && cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices) {
+                if (!P.idle[dev] && cudaStreamCreateWithFlags(&P.idle[dev], cudaStreamNonBlocking) != cudaSuccess) {
+                    P.idle[dev] = nullptr;
+                    cudaGetLastError();
+                }
+                st = P.idle[dev];
+            }
+            cudaFreeAsync(p, st);
+            return;
+        }
+    }
+    cudaFree(p);   // waits for the device, as the work on `st` needs
 }
 
 cudaError_t AcquireStream(cudaStream_t *st) {

@@ -15,8 +15,16 @@ namespace az {
 // most kPoolKept unused bytes across synchronisations; the rest goes back to
 // the driver.  Safe with several threads and streams.
 constexpr size_t kPoolKept = (size_t)2 << 30;
+// Larger buffers are cudaMalloc's: the pool maps new memory at 7.3 ms per GiB
+// and cannot keep much of a wave of tens of millions of samples, while
+// cudaMalloc and cudaFree take 0.4 ms each for 128 MiB (the pool's growth 0.95)
+// and 0.9 ms for 1 GiB.  A scene's queues live as long as the scene; what comes
+// and goes with a call is smaller (one-shot image of 230 k samples: 48 MB the
+// largest, a build of 1.3 M triangles: 62 MB).
+constexpr size_t kPoolLargest = (size_t)128 << 20;
 cudaError_t PoolAlloc(void **p, size_t bytes, cudaStream_t st);
-// Gives memory back once the work queued on `st` so far has finished.
+// Gives memory back once the work queued on `st` so far has finished; no
+// stream: when nothing uses the memory any more.
 void PoolFree(void *p, cudaStream_t st);
 
 // An array of the pool that lives as long as this object, used on one stream.
