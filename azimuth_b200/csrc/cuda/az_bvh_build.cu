@@ -248,93 +248,303 @@ __device__ __forceinline__ float merged_area(float4 alo, float4 ahi, float4 blo,
     return dx * dy + dy * dz + dz * dx;
 }
 
+// Where the rounds stand, on the device: a batch of rounds is queued without
+// the host knowing the counts between them.
+struct PlocState {
+    uint32_t count;    // clusters
+    uint32_t made;     // nodes made so far
+    uint32_t side;     // which of the two cluster arrays holds them
+    uint32_t pad;
+};
+
 __global__ void k_ploc_init(const uint32_t *order, const float4 *plo, const float4 *phi, uint32_t n, uint32_t *ids,
-                            float4 *lo, float4 *hi) {
+                            float4 *lo, float4 *hi, PlocState *start) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
+    if (i == 0) *start = PlocState{n, 0u, 0u, 0u};
     ids[i] = kLeafBit | i;   // leaf: its sorted position
     lo[i] = plo[order[i]];
     hi[i] = phi[order[i]];
-}
-
-__global__ void k_ploc_nn(const float4 *lo, const float4 *hi, uint32_t count, int radius, uint32_t *nn) {
-    const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    if (i >= (int)count) return;
-    const float4 a0 = lo[i], a1 = hi[i];
-    float best = FLT_MAX;
-    int bj = i == 0 ? 1 : i - 1;
-    const int j0 = max(0, i - radius), j1 = min((int)count - 1, i + radius);
-    for (int j = j0; j <= j1; j++) {
-        if (j == i) continue;
-        const float a = merged_area(a0, a1, __ldg(lo + j), __ldg(hi + j));
-        if (a < best) {
-            best = a;
-            bj = j;
-        }
-    }
-    nn[i] = (uint32_t)bj;
-}
-
-// Per cluster: bit 32 "creates a node" (mutual pair, lower position), bit 0 "survives".
-__global__ void k_ploc_flags(const uint32_t *nn, uint32_t count, unsigned long long *flags) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    const uint32_t j = nn[i];
-    const bool mutual = nn[j] == i;
-    flags[i] = ((unsigned long long)(mutual && i < j) << 32) | (unsigned long long)!(mutual && i > j);
 }
 
 __device__ __forceinline__ uint32_t cluster_count(uint32_t id, const uint32_t *node_count) {
     return (id & kLeafBit) ? 1u : node_count[id];
 }
 
-__global__ void k_ploc_merge(const uint32_t *ids, const float4 *lo, const float4 *hi, const uint32_t *nn,
-                             uint32_t count, const unsigned long long *flags, const unsigned long long *incl,
-                             uint32_t node_begin, uint32_t *new_ids, float4 *new_lo, float4 *new_hi,
-                             uint32_t *node_left, uint32_t *node_right, float4 *node_lo, float4 *node_hi,
-                             uint32_t *node_count) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    const unsigned long long f = flags[i];
-    if (!(f & 1ull)) return;   // merged into its lower neighbour's node
-    const unsigned long long ex = incl[i] - f;
-    const uint32_t pos = (uint32_t)(ex & 0xFFFFFFFFull);
-    if (f >> 32) {
-        const uint32_t j = nn[i], id = node_begin + (uint32_t)(ex >> 32);
-        const uint32_t a = ids[i], b = ids[j];
-        const float4 alo = lo[i], ahi = hi[i], blo = lo[j], bhi = hi[j];
-        const float4 ulo = make_float4(fminf(alo.x, blo.x), fminf(alo.y, blo.y), fminf(alo.z, blo.z), 0.0f);
-        const float4 uhi = make_float4(fmaxf(ahi.x, bhi.x), fmaxf(ahi.y, bhi.y), fmaxf(ahi.z, bhi.z), 0.0f);
-        node_left[id] = a;
-        node_right[id] = b;
-        node_lo[id] = ulo;
-        node_hi[id] = uhi;
-        node_count[id] = cluster_count(a, node_count) + cluster_count(b, node_count);
-        new_ids[pos] = id;
-        new_lo[pos] = ulo;
-        new_hi[pos] = uhi;
-    } else {
-        new_ids[pos] = ids[i];
-        new_lo[pos] = lo[i];
-        new_hi[pos] = hi[i];
+struct PlocClusters {
+    uint32_t *ids[2];
+    float4 *lo[2], *hi[2];
+};
+struct PlocNodes {
+    uint32_t *left, *right, *count;
+    float4 *lo, *hi;
+};
+
+// The neighbour of cluster i among 0..count-1 with the smallest merged box;
+// `at` reads a cluster's box.
+template <typename AT>
+__device__ __forceinline__ int ploc_nearest(int i, int count, AT at) {
+    float4 a0, a1;
+    at(i, a0, a1);
+    float best = FLT_MAX;
+    int bj = i == 0 ? 1 : i - 1;
+    const int j0 = max(0, i - kPlocRadius), j1 = min(count - 1, i + kPlocRadius);
+    for (int j = j0; j <= j1; j++) {
+        if (j == i) continue;
+        float4 b0, b1;
+        at(j, b0, b1);
+        const float a = merged_area(a0, a1, b0, b1);
+        if (a < best) {
+            best = a;
+            bj = j;
+        }
+    }
+    return bj;
+}
+
+// Node `id` from clusters a and b; its box goes to ulo, uhi.
+__device__ __forceinline__ void ploc_node(const PlocNodes &N, uint32_t id, uint32_t a, uint32_t b, float4 alo, float4 ahi,
+                                          float4 blo, float4 bhi, float4 &ulo, float4 &uhi) {
+    ulo = make_float4(fminf(alo.x, blo.x), fminf(alo.y, blo.y), fminf(alo.z, blo.z), 0.0f);
+    uhi = make_float4(fmaxf(ahi.x, bhi.x), fmaxf(ahi.y, bhi.y), fmaxf(ahi.z, bhi.z), 0.0f);
+    N.left[id] = a;
+    N.right[id] = b;
+    N.lo[id] = ulo;
+    N.hi[id] = uhi;
+    N.count[id] = cluster_count(a, N.count) + cluster_count(b, N.count);
+}
+
+// A round takes two launches.  k_ploc_pairs finds every cluster's neighbour
+// and counts the block's new nodes and survivors (bits 32.. and 0..31 of a
+// block's word).  A pair is mutual when the neighbour's neighbour is the
+// cluster itself, so the block also searches for the kPlocRadius clusters on
+// either side of its own, from boxes in shared memory.  k_ploc_merge adds the
+// words of the blocks before its own, which replaces a scan of all clusters.
+// The tree of 1.3 M triangles takes 65 rounds of five launches and a wait for
+// the host each when searched, flagged, scanned and merged apart.
+// A count of kPlocTail or fewer is left to k_ploc_tail.
+constexpr int kPlocBlock = 512;
+constexpr uint32_t kPlocTail = 1024;
+
+__global__ void __launch_bounds__(kPlocBlock) k_ploc_pairs(PlocClusters C, const PlocState *in, uint32_t *nn,
+                                                           unsigned long long *words) {
+    constexpr int kHalo = 2 * kPlocRadius, kSpan = kPlocBlock + 2 * kHalo;
+    __shared__ float4 slo[kSpan], shi[kSpan];
+    __shared__ int snn[kPlocBlock + kHalo];
+    const PlocState s = *in;
+    const int count = (int)s.count, first = (int)(blockIdx.x * kPlocBlock);
+    if (s.count <= kPlocTail || first >= count) return;
+    const float4 *lo = C.lo[s.side], *hi = C.hi[s.side];
+    const int base = first - kHalo;               // cluster of slo[0]
+    for (int k = threadIdx.x; k < kSpan; k += kPlocBlock) {
+        const int j = base + k;
+        if (j >= 0 && j < count) {
+            slo[k] = lo[j];
+            shi[k] = hi[j];
+        }
+    }
+    __syncthreads();
+    const int nbase = first - kPlocRadius;        // cluster of snn[0]
+    for (int k = threadIdx.x; k < kPlocBlock + kHalo; k += kPlocBlock) {
+        const int j = nbase + k;
+        if (j >= 0 && j < count)
+            snn[k] = ploc_nearest(j, count, [&](int c, float4 &l, float4 &h) {
+                l = slo[c - base];
+                h = shi[c - base];
+            });
+    }
+    __syncthreads();
+    const int i = first + (int)threadIdx.x;
+    bool makes = false, survives = false;
+    if (i < count) {
+        const int j = snn[i - nbase];
+        const bool mutual = snn[j - nbase] == i;
+        makes = mutual && i < j;
+        survives = !(mutual && i > j);
+        nn[i] = (uint32_t)j | (mutual ? kLeafBit : 0u);   // the top bit: mutual
+    }
+    const uint32_t m = __syncthreads_count(makes), v = __syncthreads_count(survives);
+    if (threadIdx.x == 0) words[blockIdx.x] = ((unsigned long long)m << 32) | v;
+}
+
+__global__ void __launch_bounds__(kPlocBlock) k_ploc_merge(PlocClusters C, PlocNodes N, const PlocState *in,
+                                                           PlocState *out, const uint32_t *nn,
+                                                           const unsigned long long *words) {
+    const PlocState s = *in;
+    if (s.count <= kPlocTail) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) *out = s;
+        return;
+    }
+    const uint32_t i = blockIdx.x * kPlocBlock + threadIdx.x;
+    if (blockIdx.x * kPlocBlock >= s.count) return;
+    __shared__ unsigned long long part[kPlocBlock / 32];
+    __shared__ uint32_t wmakes[kPlocBlock / 32], wsurvives[kPlocBlock / 32];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    // nodes and survivors of the blocks before this one
+    unsigned long long before = 0;
+    for (uint32_t b = threadIdx.x; b < blockIdx.x; b += kPlocBlock) before += words[b];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xFFFFFFFFu, before, o);
+    // and of the threads before this one
+    const uint32_t w = i < s.count ? nn[i] : 0u, j = w & ~kLeafBit;
+    const bool mutual = i < s.count && (w & kLeafBit), makes = mutual && i < j,
+               survives = i < s.count && !(mutual && i > j);
+    const uint32_t mb = __ballot_sync(0xFFFFFFFFu, makes), vb = __ballot_sync(0xFFFFFFFFu, survives);
+    if (lane == 0) {
+        part[warp] = before;
+        wmakes[warp] = __popc(mb);
+        wsurvives[warp] = __popc(vb);
+    }
+    __syncthreads();
+    before = 0;
+    uint32_t id = s.made + __popc(mb & ((1u << lane) - 1u)), pos = __popc(vb & ((1u << lane) - 1u));
+    for (uint32_t k = 0; k < kPlocBlock / 32; k++) {
+        before += part[k];
+        if (k < warp) {
+            id += wmakes[k];
+            pos += wsurvives[k];
+        }
+    }
+    id += (uint32_t)(before >> 32);
+    pos += (uint32_t)(before & 0xFFFFFFFFull);
+    if (i == s.count - 1) {   // the last cluster: what this round made and left
+        out->count = pos + (survives ? 1u : 0u);
+        out->made = id + (makes ? 1u : 0u);
+        out->side = s.side ^ 1u;
+    }
+    if (!survives) return;   // merged into its lower neighbour's node
+    const uint32_t *ids = C.ids[s.side];
+    const float4 *lo = C.lo[s.side], *hi = C.hi[s.side];
+    uint32_t c = ids[i];
+    float4 l = lo[i], h = hi[i];
+    if (makes) {
+        float4 ul, uh;
+        ploc_node(N, id, c, ids[j], l, h, lo[j], hi[j], ul, uh);
+        c = id;
+        l = ul;
+        h = uh;
+    }
+    C.ids[s.side ^ 1u][pos] = c;
+    C.lo[s.side ^ 1u][pos] = l;
+    C.hi[s.side ^ 1u][pos] = h;
+}
+
+// The last rounds, of at most kPlocTail clusters, by one block: a thread per
+// cluster, boxes in shared memory.  Half of a large tree's rounds are here,
+// and each is a few microseconds of latency instead of launches.
+// rounds[0] = their number, then the nodes made before each and after the last;
+// *out = the end.
+__global__ void __launch_bounds__(kPlocTail) k_ploc_tail(PlocClusters C, PlocNodes N, const PlocState *in,
+                                                         PlocState *out, uint32_t *rounds) {
+    __shared__ float4 slo[kPlocTail], shi[kPlocTail];
+    __shared__ uint32_t sid[kPlocTail];
+    __shared__ uint16_t snn[kPlocTail];
+    __shared__ uint32_t wmakes[kPlocTail / 32], wsurvives[kPlocTail / 32];
+    const PlocState s = *in;
+    const uint32_t i = threadIdx.x, warp = i >> 5, lane = i & 31u;
+    uint32_t count = s.count, made = s.made, done = 0;
+    if (count > kPlocTail) return;   // the host saw no progress
+    uint32_t c = 0;
+    float4 l = make_float4(0.0f, 0.0f, 0.0f, 0.0f), h = l;
+    if (i < count) {
+        c = C.ids[s.side][i];
+        l = C.lo[s.side][i];
+        h = C.hi[s.side][i];
+    }
+    while (count > 1) {
+        if (i < count) {
+            sid[i] = c;
+            slo[i] = l;
+            shi[i] = h;
+        }
+        __syncthreads();
+        int j = 0;
+        if (i < count) {
+            j = ploc_nearest((int)i, (int)count, [&](int k, float4 &bl, float4 &bh) {
+                bl = slo[k];
+                bh = shi[k];
+            });
+            snn[i] = (uint16_t)j;
+        }
+        __syncthreads();
+        const bool mutual = i < count && snn[j] == i, makes = mutual && (int)i < j,
+                   survives = i < count && !(mutual && (int)i > j);
+        const uint32_t mb = __ballot_sync(0xFFFFFFFFu, makes), vb = __ballot_sync(0xFFFFFFFFu, survives);
+        if (lane == 0) {
+            wmakes[warp] = __popc(mb);
+            wsurvives[warp] = __popc(vb);
+        }
+        __syncthreads();
+        uint32_t id = made + __popc(mb & ((1u << lane) - 1u)), pos = __popc(vb & ((1u << lane) - 1u));
+        uint32_t nm = 0, nv = 0;
+        for (uint32_t k = 0; k < kPlocTail / 32; k++) {
+            if (k == warp) {
+                id += nm;
+                pos += nv;
+            }
+            nm += wmakes[k];
+            nv += wsurvives[k];
+        }
+        if (makes) {
+            float4 ul, uh;
+            ploc_node(N, id, c, sid[j], l, h, slo[j], shi[j], ul, uh);
+            c = id;
+            l = ul;
+            h = uh;
+        }
+        __syncthreads();   // every box and node of this round has been read and written
+        if (i == 0) rounds[1 + done] = made;
+        if (survives) {
+            sid[pos] = c;
+            slo[pos] = l;
+            shi[pos] = h;
+        }
+        __syncthreads();
+        done++;
+        if (nm == 0) break;   // no progress: the node count tells the host
+        made += nm;
+        count = nv;
+        if (i < count) {
+            c = sid[i];
+            l = slo[i];
+            h = shi[i];
+        }
+        __syncthreads();
+    }
+    if (i == 0) {
+        rounds[0] = done;
+        rounds[1 + done] = made;
+        *out = PlocState{count, made, 0u, 0u};
     }
 }
 
 // Depth-first positions, top-down one merge round at a time (a node's parent
 // was made in a later round): the left child starts where its parent does,
 // the right child after the left child's primitives.
-__global__ void k_ploc_first(uint32_t node_begin, uint32_t nodes, const uint32_t *node_left,
-                             const uint32_t *node_right, const uint32_t *node_count, uint32_t *node_first,
-                             uint32_t *leaf_first) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nodes) return;
-    const uint32_t id = node_begin + k, f = node_first[id];
-    const uint32_t a = node_left[id], b = node_right[id];
-    const uint32_t fb = f + cluster_count(a, node_count);
+__device__ __forceinline__ void ploc_first(uint32_t id, const PlocNodes &N, uint32_t *node_first, uint32_t *leaf_first) {
+    const uint32_t f = node_first[id];
+    const uint32_t a = N.left[id], b = N.right[id];
+    const uint32_t fb = f + cluster_count(a, N.count);
     if (a & kLeafBit) leaf_first[a & ~kLeafBit] = f;
     else node_first[a] = f;
     if (b & kLeafBit) leaf_first[b & ~kLeafBit] = fb;
     else node_first[b] = fb;
+}
+
+__global__ void k_ploc_first(uint32_t node_begin, uint32_t nodes, PlocNodes N, uint32_t *node_first,
+                             uint32_t *leaf_first) {
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < nodes) ploc_first(node_begin + k, N, node_first, leaf_first);
+}
+
+// The rounds of k_ploc_tail, by one block.
+__global__ void __launch_bounds__(kPlocTail) k_ploc_first_tail(const uint32_t *rounds, PlocNodes N, uint32_t *node_first,
+                                                               uint32_t *leaf_first) {
+    for (uint32_t r = rounds[0]; r-- > 0;) {
+        const uint32_t id = rounds[1 + r] + threadIdx.x;
+        if (id < rounds[2 + r]) ploc_first(id, N, node_first, leaf_first);
+        __syncthreads();   // the nodes below read what this round wrote
+    }
 }
 
 __global__ void k_ploc_emit(uint32_t n_nodes, const uint32_t *node_left, const uint32_t *node_right,
@@ -396,11 +606,13 @@ int BuildPLOC(const float4 *d_lo, const float4 *d_hi, uint32_t n, azd::BVHNode *
               uint32_t node_base, uint32_t leaf_base, uint32_t *d_perm, cudaStream_t stream, uint32_t *root_out) {
     if (n <= 2) return BuildLBVH(d_lo, d_hi, n, d_nodes, d_range, node_base, leaf_base, d_perm, stream, root_out);
     PoolBuf<float> bounds;
-    PoolBuf<unsigned long long> keys, keys_sorted, flags, incl;
-    PoolBuf<uint32_t> vals, order, ids_a, ids_b, nn, nl, nr, ncount, nfirst, lfirst;
+    PoolBuf<unsigned long long> keys, keys_sorted, words;
+    PoolBuf<uint32_t> vals, order, ids_a, ids_b, nn, nl, nr, ncount, nfirst, lfirst, tail;
     PoolBuf<float4> lo_a, hi_a, lo_b, hi_b, nlo, nhi;
-    PoolBuf<unsigned char> temp, temp2;
+    PoolBuf<unsigned char> temp;
     PoolBuf<uint32_t> err;
+    PoolBuf<PlocState> state;
+    constexpr uint32_t kBatch = 8;   // rounds queued before the host looks at the count
     AZ_CUDA_TRY(err.alloc(1, stream));
     AZ_CUDA_TRY(cudaMemsetAsync(err.p, 0, sizeof(uint32_t), stream));
     AZ_CUDA_TRY(bounds.alloc(kBoundsFloats, stream));
@@ -415,8 +627,7 @@ int BuildPLOC(const float4 *d_lo, const float4 *d_hi, uint32_t n, azd::BVHNode *
     AZ_CUDA_TRY(lo_b.alloc(n, stream));
     AZ_CUDA_TRY(hi_b.alloc(n, stream));
     AZ_CUDA_TRY(nn.alloc(n, stream));
-    AZ_CUDA_TRY(flags.alloc(n, stream));
-    AZ_CUDA_TRY(incl.alloc(n, stream));
+    AZ_CUDA_TRY(words.alloc(n / kPlocBlock + 1, stream));
     AZ_CUDA_TRY(nl.alloc(n, stream));
     AZ_CUDA_TRY(nr.alloc(n, stream));
     AZ_CUDA_TRY(nlo.alloc(n, stream));
@@ -424,54 +635,60 @@ int BuildPLOC(const float4 *d_lo, const float4 *d_hi, uint32_t n, azd::BVHNode *
     AZ_CUDA_TRY(ncount.alloc(n, stream));
     AZ_CUDA_TRY(nfirst.alloc(n, stream));
     AZ_CUDA_TRY(lfirst.alloc(n, stream));
-    size_t temp_bytes = 0, temp2_bytes = 0;
+    AZ_CUDA_TRY(tail.alloc(kPlocTail + 2, stream));
+    AZ_CUDA_TRY(state.alloc(kBatch + 1, stream));
+    size_t temp_bytes = 0;
     AZ_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, keys.p, keys_sorted.p, vals.p, order.p, (int)n, 0,
                                                 63, stream));
     AZ_CUDA_TRY(temp.alloc(temp_bytes, stream));
-    AZ_CUDA_TRY(cub::DeviceScan::InclusiveSum(nullptr, temp2_bytes, flags.p, incl.p, (int)n, stream));
-    AZ_CUDA_TRY(temp2.alloc(temp2_bytes, stream));
     const int B = 256;
     CentreBounds(d_lo, d_hi, n, bounds.p, stream);
     k_morton<<<(n + B - 1) / B, B, 0, stream>>>(d_lo, d_hi, n, bounds.p, keys.p, vals.p);
     AZ_CUDA_TRY(cudaGetLastError());
     AZ_CUDA_TRY(cub::DeviceRadixSort::SortPairs(temp.p, temp_bytes, keys.p, keys_sorted.p, vals.p, order.p, (int)n, 0,
                                                 63, stream));
-    k_ploc_init<<<(n + B - 1) / B, B, 0, stream>>>(order.p, d_lo, d_hi, n, ids_a.p, lo_a.p, hi_a.p);
+    // state[k] is where round k of a batch starts; the last round's end is the
+    // next batch's start
+    k_ploc_init<<<(n + B - 1) / B, B, 0, stream>>>(order.p, d_lo, d_hi, n, ids_a.p, lo_a.p, hi_a.p, state.p + kBatch);
     AZ_CUDA_TRY(cudaGetLastError());
+    const PlocClusters C{{ids_a.p, ids_b.p}, {lo_a.p, lo_b.p}, {hi_a.p, hi_b.p}};
+    const PlocNodes N{nl.p, nr.p, ncount.p, nlo.p, nhi.p};
     std::vector<std::pair<uint32_t, uint32_t>> rounds;   // nodes made per round: (first id, count)
     uint32_t count = n, made = 0;
-    uint32_t *ids = ids_a.p, *ids2 = ids_b.p;
-    float4 *lo = lo_a.p, *hi = hi_a.p, *lo2 = lo_b.p, *hi2 = hi_b.p;
-    for (int round = 0; count > 1; round++) {
-        if (round > (int)n) return SetError(AZ_ERR_CUDA, "PLOC made no progress");
-        const uint32_t grid = (count + B - 1) / B;
-        k_ploc_nn<<<grid, B, 0, stream>>>(lo, hi, count, kPlocRadius, nn.p);
-        k_ploc_flags<<<grid, B, 0, stream>>>(nn.p, count, flags.p);
+    while (count > kPlocTail) {
+        const uint32_t grid = (count + kPlocBlock - 1) / kPlocBlock;   // a later round's clusters are fewer
+        for (uint32_t k = 0; k < kBatch; k++) {
+            const PlocState *in = state.p + (k == 0 ? kBatch : k);
+            k_ploc_pairs<<<grid, kPlocBlock, 0, stream>>>(C, in, nn.p, words.p);
+            k_ploc_merge<<<grid, kPlocBlock, 0, stream>>>(C, N, in, state.p + k + 1, nn.p, words.p);
+        }
         AZ_CUDA_TRY(cudaGetLastError());
-        AZ_CUDA_TRY(cub::DeviceScan::InclusiveSum(temp2.p, temp2_bytes, flags.p, incl.p, (int)count, stream));
-        k_ploc_merge<<<grid, B, 0, stream>>>(ids, lo, hi, nn.p, count, flags.p, incl.p, made, ids2, lo2, hi2, nl.p, nr.p,
-                                            nlo.p, nhi.p, ncount.p);
-        AZ_CUDA_TRY(cudaGetLastError());
-        unsigned long long tot = 0;
-        AZ_CUDA_TRY(cudaMemcpyAsync(&tot, incl.p + (count - 1), sizeof(tot), cudaMemcpyDeviceToHost, stream));
+        PlocState after[kBatch];
+        AZ_CUDA_TRY(cudaMemcpyAsync(after, state.p + 1, sizeof(after), cudaMemcpyDeviceToHost, stream));
         AZ_CUDA_TRY(cudaStreamSynchronize(stream));
-        const uint32_t merges = (uint32_t)(tot >> 32), survivors = (uint32_t)(tot & 0xFFFFFFFFull);
-        if (merges == 0 || made + merges > n - 1) return SetError(AZ_ERR_CUDA, "PLOC made no progress");
-        rounds.push_back({made, merges});
-        made += merges;
-        count = survivors;
-        std::swap(ids, ids2);
-        std::swap(lo, lo2);
-        std::swap(hi, hi2);
+        for (const PlocState &a : after) {
+            if (count <= kPlocTail) break;   // this round and the rest of the batch were skipped
+            if (a.made <= made || a.made > n - 1 || a.count + (a.made - made) != count)
+                return SetError(AZ_ERR_CUDA, "PLOC made no progress");
+            rounds.push_back({made, a.made - made});
+            made = a.made;
+            count = a.count;
+        }
     }
-    if (made != n - 1) return SetError(AZ_ERR_CUDA, "PLOC did not build a binary tree");
+    k_ploc_tail<<<1, kPlocTail, 0, stream>>>(C, N, state.p + kBatch, state.p, tail.p);
+    AZ_CUDA_TRY(cudaGetLastError());
+    PlocState end{};
+    AZ_CUDA_TRY(cudaMemcpyAsync(&end, state.p, sizeof(end), cudaMemcpyDeviceToHost, stream));
+    AZ_CUDA_TRY(cudaStreamSynchronize(stream));
+    if (end.count != 1 || end.made != n - 1) return SetError(AZ_ERR_CUDA, "PLOC did not build a binary tree");
     // depth-first positions from the root (the last node made) down
     const uint32_t root = n - 2;
     AZ_CUDA_TRY(cudaMemsetAsync(nfirst.p, 0, (size_t)n * sizeof(uint32_t), stream));
     AZ_CUDA_TRY(cudaMemsetAsync(lfirst.p, 0xFF, (size_t)n * sizeof(uint32_t), stream));
+    k_ploc_first_tail<<<1, kPlocTail, 0, stream>>>(tail.p, N, nfirst.p, lfirst.p);
     for (size_t r = rounds.size(); r-- > 0;) {
         const uint32_t k = rounds[r].second;
-        k_ploc_first<<<(k + B - 1) / B, B, 0, stream>>>(rounds[r].first, k, nl.p, nr.p, ncount.p, nfirst.p, lfirst.p);
+        k_ploc_first<<<(k + B - 1) / B, B, 0, stream>>>(rounds[r].first, k, N, nfirst.p, lfirst.p);
     }
     AZ_CUDA_TRY(cudaGetLastError());
     k_ploc_emit<<<(n - 1 + B - 1) / B, B, 0, stream>>>(n - 1, nl.p, nr.p, nlo.p, nhi.p, ncount.p, nfirst.p, lfirst.p,

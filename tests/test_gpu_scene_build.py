@@ -102,3 +102,21 @@ def test_ploc_visits_fewer_nodes(gpu, dense):
             visits[builder] = (st["node_visits"] + st["prim_visits"] + st["shadow_node_visits"] +
                                st["shadow_prim_visits"]) / (st["extend_rays"] + st["shadow_rays"])
     assert visits[az.BVH_PLOC] < visits[az.BVH_LBVH]
+
+
+@pytest.mark.parametrize("spheres", [511, 512, 1023, 1024, 1025, 1537, 2049, 5001])
+def test_ploc_at_the_edges_of_its_blocks(gpu, spheres):
+    # one hierarchy of `spheres` primitives: below, at and above the last rounds'
+    # block and the blocks of a merge round
+    sc = az.generate_scene(az.SCENE_MOTION_ENV, seed=7, width=16, height=16, spp=1, detail=spheres)
+    try:
+        rays = _rays(1 << 14, seed=spheres, lo=0.0, hi=10.0)
+        with az.GpuScene(sc, bvh_builder=az.BVH_LBVH) as a, az.GpuScene(sc, bvh_builder=az.BVH_PLOC) as b:
+            assert a.info()["spheres"] == b.info()["spheres"] >= spheres
+            ha, hb = a.closest_hit(rays), b.closest_hit(rays)
+        assert ha[0].any()
+        same = (ha[0] == hb[0]) & (ha[1] == hb[1]) & (ha[3] == hb[3])
+        assert same.mean() >= 0.999
+        assert np.array_equal(ha[3][~same], hb[3][~same])   # exact-distance ties only
+    finally:
+        sc.close()
