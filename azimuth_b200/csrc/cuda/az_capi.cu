@@ -132,7 +132,7 @@ extern "C" int az_gpu_mesh_postprocess(const az_mesh_soup *soup, az_vec3 *vertex
     std::unique_ptr<SoupWork, void (*)(SoupWork *)> hold(w, FreeSoupWork);
     if (total_area) {
         std::vector<float> a;
-        if ((rc = SoupAreas(*w, a)) != AZ_OK) return rc;
+        if ((rc = SoupAreas(*w, a, ctx.stream)) != AZ_OK) return rc;
         if (!a.empty()) memcpy(total_area, a.data(), a.size() * sizeof(float));
     }
     return SoupRecords(*w, triangles, attrs, vertex_normals, ctx.stream);

@@ -74,7 +74,8 @@ struct IngestMesh {
 };
 int IngestSoup(const az_mesh_soup *soup, cudaStream_t st, SoupWork **out);
 void FreeSoupWork(SoupWork *w);
-int SoupAreas(const SoupWork &w, std::vector<float> &areas);
+int SoupAreas(const SoupWork &w, std::vector<float> &areas, cudaStream_t st);
+int SoupArea(const SoupWork &w, uint32_t mesh, float &area, cudaStream_t st);   // one mesh's
 // Per mesh (soup order): lo.xyz, hi.xyz of its faces' vertices.
 int SoupBoxes(const SoupWork &w, std::vector<float> &boxes, cudaStream_t st);
 int SoupRecords(const SoupWork &w, az_triangle *tris, az_face_attr *attrs, az_vec3 *vertex_normals, cudaStream_t st);

@@ -270,6 +270,7 @@ struct SoupWork {
     PoolBuf<float> v, uv, fn_raw, fn_unit, half_area, vn, area;
     PoolBuf<uint32_t> faces;
     PoolBuf<MeshRange> ranges;
+    std::vector<MeshRange> host_ranges;   // in the order of `ranges`
 };
 
 void FreeSoupWork(SoupWork *w) { delete w; }
@@ -347,24 +348,36 @@ int IngestSoup(const az_mesh_soup *soup, cudaStream_t st, SoupWork **out) {
                                                     end_bit, st));
         k_ingest_segments<<<(n_inc + B - 1) / B, B, 0, st>>>(skey.p, n_inc, vstart.p, vend.p);
         AZ_CUDA_TRY(cudaGetLastError());
-        AZ_CUDA_TRY(cudaStreamSynchronize(st));   // temp is freed on return
     }
     if (nv) {
         k_ingest_vertices<<<(nv + B - 1) / B, B, 0, st>>>(vstart.p, vend.p, sval.p, W->fn_raw.p, nv, W->vn.p);
         AZ_CUDA_TRY(cudaGetLastError());
     }
-    if (W->nm) {
-        k_ingest_area<<<W->nm, kAreaBlock, 0, st>>>(W->ranges.p, W->half_area.p, W->area.p);
-        AZ_CUDA_TRY(cudaGetLastError());
-    }
-    AZ_CUDA_TRY(cudaStreamSynchronize(st));
+    W->host_ranges.swap(ranges);
     *out = W.release();
     return AZ_OK;
 }
 
-int SoupAreas(const SoupWork &w, std::vector<float> &areas) {
+int SoupAreas(const SoupWork &w, std::vector<float> &areas, cudaStream_t st) {
     areas.assign(w.nm, 0.0f);
-    if (w.nm) AZ_CUDA_TRY(cudaMemcpy(areas.data(), w.area.p, w.nm * sizeof(float), cudaMemcpyDeviceToHost));
+    if (w.nm == 0) return AZ_OK;
+    k_ingest_area<<<w.nm, kAreaBlock, 0, st>>>(w.ranges.p, w.half_area.p, w.area.p);
+    AZ_CUDA_TRY(cudaGetLastError());
+    AZ_CUDA_TRY(cudaMemcpyAsync(areas.data(), w.area.p, w.nm * sizeof(float), cudaMemcpyDeviceToHost, st));
+    AZ_CUDA_TRY(cudaStreamSynchronize(st));
+    return AZ_OK;
+}
+
+int SoupArea(const SoupWork &w, uint32_t mesh, float &area, cudaStream_t st) {
+    area = 0.0f;
+    for (size_t k = 0; k < w.host_ranges.size(); k++) {
+        if (w.host_ranges[k].index != mesh) continue;
+        k_ingest_area<<<1, kAreaBlock, 0, st>>>(w.ranges.p + k, w.half_area.p, w.area.p);
+        AZ_CUDA_TRY(cudaGetLastError());
+        AZ_CUDA_TRY(cudaMemcpyAsync(&area, w.area.p + mesh, sizeof(float), cudaMemcpyDeviceToHost, st));
+        AZ_CUDA_TRY(cudaStreamSynchronize(st));
+        break;
+    }
     return AZ_OK;
 }
 
