@@ -38,7 +38,7 @@ constexpr int kPostBlock = 256;
 struct PostScratch {
     double logsum;
     float white;
-    uint32_t hist[3][kBins];
+    alignas(16) uint32_t hist[3][kBins];
 };
 
 // Keys whose unsigned order is the luminances' order (a radix sort's: negative
@@ -71,6 +71,7 @@ __global__ void __launch_bounds__(kPostBlock) k_post_luminance(const float4 *fil
     for (uint32_t b = threadIdx.x; b < kBins; b += kPostBlock) bins[b] = 0u;
     __syncthreads();
     double part = 0.0;
+#pragma unroll 4
     for (uint32_t i = blockIdx.x * kPostBlock + threadIdx.x; i < n; i += gridDim.x * kPostBlock) {
         float c[3];
         colour_of(film[i], c);
@@ -94,19 +95,27 @@ __global__ void __launch_bounds__(kPostBlock) k_post_luminance(const float4 *fil
 // within it; called by the whole block.
 __device__ __forceinline__ uint32_t pick_bin(const uint32_t *hist, uint32_t rank, uint32_t &rest) {
     constexpr uint32_t kPer = kBins / kPostBlock;
-    __shared__ uint32_t scan[kPostBlock];
+    static_assert(kPer == 8, "two 16-byte loads a thread");
+    __shared__ uint32_t warps[kPostBlock / 32];
     __shared__ uint32_t found[2];
-    uint32_t h[kPer], own = 0;
-    for (uint32_t k = 0; k < kPer; k++) own += h[k] = hist[threadIdx.x * kPer + k];
-    scan[threadIdx.x] = own;
-    __syncthreads();
-    for (uint32_t d = 1; d < kPostBlock; d <<= 1) {
-        const uint32_t v = threadIdx.x >= d ? scan[threadIdx.x - d] : 0u;
-        __syncthreads();
-        scan[threadIdx.x] += v;
-        __syncthreads();
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const uint4 *src = reinterpret_cast<const uint4 *>(hist) + 2u * threadIdx.x;
+    const uint4 h0 = src[0], h1 = src[1];
+    const uint32_t h[kPer] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+    uint32_t own = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kPer; k++) own += h[k];
+    uint32_t before = own;   // inclusive within the warp
+#pragma unroll
+    for (uint32_t d = 1; d < 32; d <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, before, d);
+        if (lane >= d) before += v;
     }
-    uint32_t before = scan[threadIdx.x] - own;
+    if (lane == 31) warps[warp] = before;
+    __syncthreads();
+    before -= own;
+    for (uint32_t w = 0; w < warp; w++) before += warps[w];
+#pragma unroll
     for (uint32_t k = 0; k < kPer; k++) {
         if (rank >= before && rank - before < h[k]) {
             found[0] = threadIdx.x * kPer + k;
@@ -122,6 +131,7 @@ __device__ __forceinline__ uint32_t pick_bin(const uint32_t *hist, uint32_t rank
 }
 
 // PASS 1 and 2: the next bits of the keys that share the selected prefix.
+// Four keys a load: with one, a thread waited for memory 14 times.
 template <int PASS>
 __global__ void __launch_bounds__(kPostBlock) k_post_histogram(const uint32_t *keys, uint32_t n, uint32_t rank,
                                                                PostScratch *S) {
@@ -130,10 +140,19 @@ __global__ void __launch_bounds__(kPostBlock) k_post_histogram(const uint32_t *k
     uint32_t rest;
     uint32_t prefix = pick_bin(S->hist[0], rank, rest);
     if (PASS == 2) prefix = prefix << 11 | pick_bin(S->hist[1], rest, rest);
-    for (uint32_t i = blockIdx.x * kPostBlock + threadIdx.x; i < n; i += gridDim.x * kPostBlock) {
-        const uint32_t k = keys[i];
+    auto count = [&](uint32_t k) {
         if (k >> (PASS == 1 ? 21 : 10) == prefix) atomicAdd(&bins[PASS == 1 ? (k >> 10) & 2047u : k & 1023u], 1u);
+    };
+    const uint32_t first = blockIdx.x * kPostBlock + threadIdx.x, step = gridDim.x * kPostBlock;
+#pragma unroll 2
+    for (uint32_t i = first; i < n / 4u; i += step) {
+        const uint4 k = reinterpret_cast<const uint4 *>(keys)[i];
+        count(k.x);
+        count(k.y);
+        count(k.z);
+        count(k.w);
     }
+    if (first < (n & 3u)) count(keys[(n & ~3u) + first]);
     add_histogram(bins, S->hist[PASS]);
 }
 
@@ -152,13 +171,18 @@ struct MapParams {
     uint32_t srgb, linear;
 };
 
+// powf(q, 1) is q for every q, NaN and infinities among them (all 2^32 were
+// tried), so the default saturation of 1 needs three powf a pixel instead of six.
 __device__ __forceinline__ void map_colour(float c[3], const MapParams &P) {
     if (P.tonemapped) {
         const float l = lum3(c[0], c[1], c[2]);
         if (l != 0.0f) {
             const float ls = l * P.factor;
             const float ld = (ls * (1.0f + (ls / P.lw2))) / (1.0f + ls);
-            for (int k = 0; k < 3; k++) c[k] = clamp01(powf(c[k] / l, P.saturation) * ld);
+            for (int k = 0; k < 3; k++) {
+                const float q = c[k] / l;
+                c[k] = clamp01((P.saturation == 1.0f ? q : powf(q, P.saturation)) * ld);
+            }
         }
     }
     if (P.linear) return;
