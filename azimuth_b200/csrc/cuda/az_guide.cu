@@ -384,10 +384,10 @@ constexpr uint32_t kTcWaitLimit = 1u << 20;   // polls of an mbarrier (a layer c
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // Shared-memory matrix descriptor (no swizzle, K-major, sm_100 version
-// field): core matrices along K 128 bytes apart, row groups `sbo` bytes apart
-// (1024 for a 64-wide K, 2048 for the 128-wide K of the transposed operands).
-__device__ __forceinline__ uint64_t tc_desc(uint32_t saddr, uint32_t sbo = 1024u) {
-    return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)(128u >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) |
+// field): core matrices along K `lbo` bytes apart, row groups `sbo` bytes apart
+// (128 and 1024 for a 64-wide K; see tc_offset_t for the transposed operands).
+__device__ __forceinline__ uint64_t tc_desc(uint32_t saddr, uint32_t sbo = 1024u, uint32_t lbo = 128u) {
+    return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) |
            ((uint64_t)1 << 46);
 }
 
@@ -432,25 +432,6 @@ __device__ __forceinline__ void tc_load16(uint32_t taddr, float *v) {
         : "r"(taddr));
 #pragma unroll
     for (int j = 0; j < 16; j++) v[j] = __uint_as_float(r[j]);
-}
-
-// Row `r` of the A operand from 64 floats (BF16, 8 chunks of 16 bytes).
-__device__ __forceinline__ void tc_store_row(unsigned char *A, uint32_t r, const float *x, bool relu) {
-#pragma unroll
-    for (int kc = 0; kc < 8; kc++) {
-        uint4 q;
-        uint32_t *u = reinterpret_cast<uint32_t *>(&q);
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            float a = x[8 * kc + 2 * j], b = x[8 * kc + 2 * j + 1];
-            if (relu) {
-                a = fmaxf(a, 0.0f);
-                b = fmaxf(b, 0.0f);
-            }
-            u[j] = pack_bf16(a, b);
-        }
-        *reinterpret_cast<uint4 *>(A + tc_offset(r, 8u * kc)) = q;
-    }
 }
 
 // Chunks KC0 .. KC0 + NKC - 1 (8 columns each) of row r of the A operand from
@@ -919,60 +900,128 @@ __global__ void __launch_bounds__(kWarps * 32) k_guide_train(GuideNetDev N, Trai
 }
 
 // ---- the same training step on the 5th-generation tensor cores (tcgen05) ----
-// One CTA of 128 threads per SM takes 128 rows at a time, one row per thread,
-// and keeps the whole step's tensor work on tcgen05.mma (M = 128, N = 64,
-// K = 16 per instruction, BF16 operands in shared memory, FP32 accumulators in
-// tensor memory):
+// One CTA of 512 threads per SM takes 128 rows at a time, four threads a row
+// (each 16 of its 64 columns, 4 of its 16 grid levels), and keeps the whole
+// step's tensor work on tcgen05.mma (M = 128, N = 64, K = 16 per instruction,
+// BF16 operands in shared memory, FP32 accumulators in tensor memory):
 //   forward   X_{l+1} = ReLU(X_l W_l), Y = X_3 W_3 + b  (A = X_l, 64-wide K)
 //   backward  dX_l = dY_l W_l^T                          (A = dY_l, 64-wide K)
 //             dW_l += X_l^T dY_l                         (K = the tile's 128 rows)
-// The dW products need the rows as K: every thread also writes its row of X_l
+// The dW products need the rows as K: every thread also writes its part of X_l
 // and dY_l into transposed operands (element (unit u, row r) at
 // tc_offset_t(u, r)).  Their M is the 64 input units; the instruction's other
-// 64 rows read the next 16 KB of shared memory and land in tensor-memory
-// lanes 64..127, which are never read.  dW_l accumulates in its own 64
-// tensor-memory columns over all the CTA's tiles in tile order, so the sums
-// do not depend on timing; after the last tile warps 0 and 1 (lanes 0..63)
-// write them to the CTA's slot of `part`, which k_guide_reduce adds up in
-// block order like the mma.sync kernel's.  Output-bias gradients and the loss
-// are summed in fixed order through shared memory; the hash-grid gradient is
-// scattered in fixed point as in k_guide_train.  Waits on the mbarrier are
-// bounded: on a timeout *err is set and the CTA stops (its slot then holds
-// what it had).
+// 64 rows read the operand that follows in shared memory and land in
+// tensor-memory lanes 64..127, which are never read.  dW_l accumulates in its
+// own 64 tensor-memory columns over all the CTA's tiles in tile order, so the
+// sums do not depend on timing; after the last tile the warps of lanes 0..63
+// write them to the CTA's slot of `part`, which is added up in block order like
+// the mma.sync kernel's.  Output-bias gradients and the loss are summed in
+// fixed order through shared memory; the hash-grid gradient is scattered in
+// fixed point as in k_guide_train.  Waits on the mbarrier are bounded: on a
+// timeout *err is set and the CTA stops (its slot then holds what it had).
+//
+// What bounds it: 128 gathers and 256 scattered 64-bit additions a row, whose
+// latency only threads can hide.  With a thread a row (4 warps an SM) the kernel
+// took 470 us on 100,003 rows at 6 % of the SM's warps (430 now; 290 of them without the scatter).
+//
+// The K direction of a transposed operand steps by 144 bytes instead of 128: a
+// warp's 32 rows are four core matrices, and at 128 bytes apart the 2-byte
+// stores of all four met in the same banks.
+constexpr uint32_t kTcLboT = 144, kTcSboT = 16 * kTcLboT;
 __host__ __device__ __forceinline__ uint32_t tc_offset_t(uint32_t u, uint32_t r) {
-    return ((u >> 3) * 16u + (r >> 3)) * 128u + (u & 7u) * 16u + (r & 7u) * 2u;
+    return (u >> 3) * kTcSboT + (r >> 3) * kTcLboT + (u & 7u) * 16u + (r & 7u) * 2u;
 }
 
+constexpr uint32_t kTcTrainThreads = 4 * kTcRows;
 constexpr uint32_t kTcOp = kTcRows * W * 2;             // bytes of one 128 x 64 BF16 operand
+constexpr uint32_t kTcOpT = W / 8 * kTcSboT;            // bytes of one transposed operand
 constexpr uint32_t kTcTrainCols = 512;                  // tensor memory: scratch + 4 dW accumulators (320 used)
-// shared memory: X (A layout), X_l^T for l = 0..3, dY (A layout), dY^T, W^T
-// and W per layer (B operands of the forward and of dX), dY in FP32 for the
-// bias gradient, bias, bias gradient, loss, mbarrier, tensor-memory address
-constexpr size_t kTcTrainSmem = (size_t)kTcOp * 7 + (size_t)NW * 2 * 2 + (size_t)kTcRows * W * sizeof(float) +
-                                2 * W * sizeof(float) + kTcRows / 32 * sizeof(float) + 16;
+constexpr uint32_t kTcOS = W + 1;                       // row stride of the FP32 outputs and their gradient: a warp's
+                                                        // 32 rows of one column in 32 banks
+// shared memory: X_l^T for l = 0..3, X (A layout), dY (A layout), dY^T, W^T
+// and W per layer (B operands of the forward and of dX), outputs then dY in
+// FP32, bias, bias gradient, loss, mbarrier, tensor-memory address
+constexpr size_t kTcTrainSmem = (size_t)kTcOpT * 5 + (size_t)kTcOp * 2 + (size_t)NW * 2 * 2 +
+                                (size_t)kTcRows * kTcOS * sizeof(float) + 2 * W * sizeof(float) +
+                                kTcRows / 32 * sizeof(float) + 16;
+static_assert(kTcTrainSmem <= 227 * 1024, "one CTA's shared memory");
 
-// this thread's row of a transposed operand (u = 0..63 at row r), as BF16
-__device__ __forceinline__ void tc_store_col(unsigned char *T, uint32_t r, const float *x) {
+// Chunks kc0 .. kc0 + NKC - 1 of row r of an A operand and of column r of its
+// transpose from x[0 .. 8 NKC), as BF16.  Returns a bit per value that is
+// positive after rounding.
+template <int NKC>
+__device__ __forceinline__ uint32_t tc_store_both(unsigned char *A, unsigned char *T, uint32_t r, uint32_t kc0,
+                                                  const float *x) {
+    uint32_t positive = 0;
 #pragma unroll
-    for (int u = 0; u < W; u++)
-        *reinterpret_cast<__nv_bfloat16 *>(T + tc_offset_t((uint32_t)u, r)) = __float2bfloat16_rn(x[u]);
+    for (int c = 0; c < NKC; c++) {
+        uint4 q;
+        uint32_t *u = reinterpret_cast<uint32_t *>(&q);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            u[j] = pack_bf16(x[8 * c + 2 * j], x[8 * c + 2 * j + 1]);
+            const float2 v = unpack_bf16(u[j]);
+            if (v.x > 0.0f) positive |= 1u << (8 * c + 2 * j);
+            if (v.y > 0.0f) positive |= 2u << (8 * c + 2 * j);
+            unsigned char *t = T + tc_offset_t(8u * (kc0 + c) + 2 * j, r);
+            *reinterpret_cast<unsigned short *>(t) = (unsigned short)(u[j] & 0xFFFFu);
+            *reinterpret_cast<unsigned short *>(t + 16) = (unsigned short)(u[j] >> 16);   // the next unit
+        }
+        *reinterpret_cast<uint4 *>(A + tc_offset(r, 8u * (kc0 + c))) = q;
+    }
+    return positive;
 }
 
-__global__ void __launch_bounds__(kTcRows, 1) k_guide_train_tc(GuideNetDev N, TrainArgs A, uint32_t *err) {
+// 8 consecutive accumulator columns of this thread's lane.
+__device__ __forceinline__ void tc_load8(uint32_t taddr, float *v) {
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
+#pragma unroll
+    for (int j = 0; j < 8; j++) v[j] = __uint_as_float(r[j]);
+}
+
+// Adds (gx, gy) times the corner weights of this lane's row to the grid
+// gradient; called by all 32 lanes.  The two sums of an entry are neighbours:
+// lanes 2k and 2k + 1 add the first and the second sum of one row's corner,
+// then of the other row's, so that an instruction touches an entry's 16 bytes
+// once instead of two instructions touching them apart.
+__device__ __forceinline__ void scatter_level(const GuideNetDev &N, unsigned long long *grad, int l, f3 p, bool live,
+                                              float gx, float gy) {
+    constexpr uint32_t kAll = 0xFFFFFFFFu;
+    const bool odd = threadIdx.x & 1u;
+    const bool live_other = __shfl_xor_sync(kAll, (int)live, 1);
+    const bool live_first = odd ? live_other : live, live_second = odd ? live : live_other;
+    Corners c;
+    grid_corners(N, l, p, c);
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const unsigned long long vx = to_fixed(c.w[k] * gx), vy = to_fixed(c.w[k] * gy);
+        const uint32_t other = __shfl_xor_sync(kAll, c.idx[k], 1);
+        const unsigned long long sent = __shfl_xor_sync(kAll, odd ? vx : vy, 1);
+        const unsigned long long first = odd ? sent : vx, second = odd ? vy : sent;
+        if (live_first && first) atomicAdd(&grad[2 * (size_t)(odd ? other : c.idx[k]) + odd], first);
+        if (live_second && second) atomicAdd(&grad[2 * (size_t)(odd ? c.idx[k] : other) + odd], second);
+    }
+}
+
+__global__ void __launch_bounds__(kTcTrainThreads, 1) k_guide_train_tc(GuideNetDev N, TrainArgs A, uint32_t *err) {
     extern __shared__ __align__(16) unsigned char smem[];
-    unsigned char *XA = smem;                      // X_l, rows (A operand of the forward)
-    unsigned char *XT = XA + kTcOp;                // X_l^T, l = 0..3
-    unsigned char *DYA = XT + 4 * kTcOp;           // dY_l, rows (A operand of dX)
+    unsigned char *XT = smem;                      // X_l^T, l = 0..3
+    unsigned char *XA = XT + 4 * kTcOpT;           // X_l, rows (A operand of the forward)
+    unsigned char *DYA = XA + kTcOp;               // dY_l, rows (A operand of dX)
     unsigned char *DYT = DYA + kTcOp;              // dY_l^T (B operand of dW)
-    unsigned char *WF = DYT + kTcOp;               // per layer W^T: row = output unit (forward)
+    unsigned char *WF = DYT + kTcOpT;              // per layer W^T: row = output unit (forward)
     unsigned char *WB = WF + NW * 2;               // per layer W: row = input unit (dX)
-    float *s_o = reinterpret_cast<float *>(WB + NW * 2);   // [128][64] dY in FP32
-    float *s_bias = s_o + kTcRows * W;
+    float *s_o = reinterpret_cast<float *>(WB + NW * 2);   // [128][kTcOS]
+    float *s_bias = s_o + kTcRows * kTcOS;
     float *s_db = s_bias + W;
     float *s_loss = s_db + W;
     uint64_t *s_mbar = reinterpret_cast<uint64_t *>(s_loss + kTcRows / 32);
     uint32_t *s_tmem = reinterpret_cast<uint32_t *>(s_mbar + 1);
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+    const uint32_t r = tid & (kTcRows - 1u), q = tid / kTcRows;   // row of the tile, which quarter of it
     {
         const uint4 *src = reinterpret_cast<const uint4 *>(N.wtc);
         uint4 *dst = reinterpret_cast<uint4 *>(WF);
@@ -998,7 +1047,7 @@ __global__ void __launch_bounds__(kTcRows, 1) k_guide_train_tc(GuideNetDev N, Tr
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *s_tmem;
-    const uint32_t lane_addr = (32u * warp) << 16;
+    const uint32_t lane_addr = (32u * (warp & 3u)) << 16;   // the warps of a row's quarters share its lanes
     const uint32_t sXA = smem_u32(XA), sXT = smem_u32(XT), sDYA = smem_u32(DYA), sDYT = smem_u32(DYT),
                    sWF = smem_u32(WF), sWB = smem_u32(WB);
     const uint32_t n = min(*A.count, A.cap);
@@ -1029,117 +1078,117 @@ __global__ void __launch_bounds__(kTcRows, 1) k_guide_train_tc(GuideNetDev N, Tr
         return true;
     };
     for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-        const uint32_t i = tile * kTcRows + tid;
+        const uint32_t i = tile * kTcRows + r;
+        const bool live = i < n;
         f3 p = mk(0.0f, 0.0f, 1.0f), nr = p, wo = p;
         GuideRow row;
-        if (i < n) {
+        if (live) {
             row = A.rows[i];
             p = normalise_pos(N, mk(row.pos_w.x, row.pos_w.y, row.pos_w.z));
             nr = mk(row.n.x, row.n.y, row.n.z);
             wo = mk(row.wo.x, row.wo.y, row.wo.z);
         }
-        float x[W];
+        float x[16];
+        uint32_t positive[GUIDE_LAYERS];   // X_l > 0, this thread's 16 columns
+        // ---- inputs: grid levels 4 q .. 4 q + 3, and 8 of the other columns ----
 #pragma unroll
-        for (int l = 0; l < GUIDE_LEVELS; l++) {
-            const float2 f = grid_feature(N, l, p);
+        for (int l = 0; l < GUIDE_LEVELS / 4; l++) {
+            const float2 f = grid_feature(N, l + (int)q * (GUIDE_LEVELS / 4), p);
             x[2 * l] = f.x;
             x[2 * l + 1] = f.y;
         }
-        x[32] = nr.x; x[33] = nr.y; x[34] = nr.z;
-        x[35] = wo.x; x[36] = wo.y; x[37] = wo.z;
-        x[38] = 1.0f;
+        tc_store_both<1>(XA, XT, r, q, x);
 #pragma unroll
-        for (int j = 39; j < W; j++) x[j] = 0.0f;
-        tc_store_row(XA, tid, x, false);
-        tc_store_col(XT, tid, x);
+        for (int j = 0; j < 8; j++) x[j] = 0.0f;
+        if (q == 0) {
+            x[0] = nr.x; x[1] = nr.y; x[2] = nr.z;
+            x[3] = wo.x; x[4] = wo.y; x[5] = wo.z;
+            x[6] = 1.0f;
+        }
+        tc_store_both<1>(XA, XT, r, 4u + q, x);
         // ---- forward ----
-        for (int l = 0; l < GUIDE_LAYERS && ok; l++) {
+#pragma unroll
+        for (int l = 0; l < GUIDE_LAYERS; l++) {
             ok = sync_issue_wait([&] {
 #pragma unroll
                 for (uint32_t ks = 0; ks < (uint32_t)W / 16; ks++)
                     tc_mma(tmem, tc_desc(sXA + ks * 256u), tc_desc(sWF + (uint32_t)l * W * W * 2 + ks * 256u), ks);
             });
             if (!ok) break;
-#pragma unroll
-            for (int c = 0; c < 4; c++) tc_load16(tmem + lane_addr + 16u * c, x + 16 * c);
+            tc_load16(tmem + lane_addr + 16u * q, x);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             if (l + 1 < GUIDE_LAYERS) {
 #pragma unroll
-                for (int j = 0; j < W; j++) x[j] = fmaxf(x[j], 0.0f);
-                tc_store_row(XA, tid, x, false);
-                tc_store_col(XT + (l + 1) * kTcOp, tid, x);
+                for (int j = 0; j < 16; j++) x[j] = fmaxf(x[j], 0.0f);
+                positive[l + 1] = tc_store_both<2>(XA, XT + (l + 1) * kTcOpT, r, 2u * q, x);
             }
         }
         if (!ok) break;
-        // ---- loss and output gradient of this thread's row ----
+        // ---- loss and output gradient: a thread a row, in place ----
+        float *o = s_o + r * kTcOS;
 #pragma unroll
-        for (int j = 0; j < W; j++) x[j] += s_bias[j];
-        if (A.dbg_out && i < n)
-            for (int j = 0; j < W; j++) A.dbg_out[(size_t)i * W + j] = x[j];
-        float d[W];
-        if (i < n) {
-            loss_acc += loss_grad(x, mk(row.n.x, row.n.y, row.n.z), mk(row.wi.x, row.wi.y, row.wi.z),
-                                  fminf(row.pos_w.w * wscale, wcap), d);
-        } else {
-#pragma unroll
-            for (int j = 0; j < W; j++) d[j] = 0.0f;
+        for (int j = 0; j < 16; j++) {
+            x[j] += s_bias[16 * q + j];
+            o[16 * q + j] = x[j];
         }
+        if (A.dbg_out && live)
+            for (int j = 0; j < 16; j++) A.dbg_out[(size_t)i * W + 16 * q + j] = x[j];
+        __syncthreads();
+        if (q == 0) {
+            if (live) {
+                loss_acc += loss_grad(o, mk(row.n.x, row.n.y, row.n.z), mk(row.wi.x, row.wi.y, row.wi.z),
+                                      fminf(row.pos_w.w * wscale, wcap), o);
+            } else {
+                for (int j = 0; j < W; j++) o[j] = 0.0f;
+            }
+        }
+        __syncthreads();
 #pragma unroll
-        for (int j = 0; j < W; j++) s_o[tid * W + j] = d[j];
-        tc_store_row(DYA, tid, d, false);
-        tc_store_col(DYT, tid, d);
+        for (int j = 0; j < 16; j++) x[j] = o[16 * q + j];
+        tc_store_both<2>(DYA, DYT, r, 2u * q, x);
         // ---- backward ----
-        for (int l = GUIDE_LAYERS - 1; l >= 0 && ok; l--) {
+#pragma unroll
+        for (int l = GUIDE_LAYERS - 1; l >= 0; l--) {
             const bool acc = has_acc;
             ok = sync_issue_wait([&] {
                 // dW_l (+)= X_l^T dY_l over this tile's rows
 #pragma unroll
                 for (uint32_t ks = 0; ks < kTcRows / 16; ks++)
-                    tc_mma(tmem + 64u * (uint32_t)(l + 1), tc_desc(sXT + (uint32_t)l * kTcOp + ks * 256u, 2048u),
-                           tc_desc(sDYT + ks * 256u, 2048u), (acc || ks) ? 1u : 0u);
+                    tc_mma(tmem + 64u * (uint32_t)(l + 1),
+                           tc_desc(sXT + (uint32_t)l * kTcOpT + ks * 2u * kTcLboT, kTcSboT, kTcLboT),
+                           tc_desc(sDYT + ks * 2u * kTcLboT, kTcSboT, kTcLboT), (acc || ks) ? 1u : 0u);
                 // dX_l = dY_l W_l^T
 #pragma unroll
                 for (uint32_t ks = 0; ks < (uint32_t)W / 16; ks++)
                     tc_mma(tmem, tc_desc(sDYA + ks * 256u), tc_desc(sWB + (uint32_t)l * W * W * 2 + ks * 256u), ks);
             });
             if (!ok) break;
-            if (l == GUIDE_LAYERS - 1 && tid < (uint32_t)W) {
-                // output-bias gradient: thread j sums column j over the rows in order
-                float s = 0.0f;
-                for (uint32_t r = 0; r < kTcRows; r++) s += s_o[r * W + tid];
-                s_db[tid] += s;
-            }
-#pragma unroll
-            for (int c = 0; c < 4; c++) tc_load16(tmem + lane_addr + 16u * c, x + 16 * c);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             if (l > 0) {
+                tc_load16(tmem + lane_addr + 16u * q, x);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 // through the ReLU that produced X_l: dY_{l-1} = dX_l where X_l > 0
-                const unsigned char *T = XT + l * kTcOp;
 #pragma unroll
-                for (int u = 0; u < W; u++) {
-                    const float xv = __bfloat162float(
-                        *reinterpret_cast<const __nv_bfloat16 *>(T + tc_offset_t((uint32_t)u, tid)));
-                    d[u] = xv > 0.0f ? x[u] : 0.0f;
+                for (int j = 0; j < 16; j++) x[j] = (positive[l] >> j) & 1u ? x[j] : 0.0f;
+                tc_store_both<2>(DYA, DYT, r, 2u * q, x);
+                if (l == GUIDE_LAYERS - 1 && q == 3 && r < (uint32_t)W) {
+                    // output-bias gradient: thread j sums column j over the rows in order
+                    float s = 0.0f;
+#pragma unroll 16
+                    for (uint32_t k = 0; k < kTcRows; k++) s += s_o[k * kTcOS + r];
+                    s_db[r] += s;
                 }
-                tc_store_row(DYA, tid, d, false);
-                tc_store_col(DYT, tid, d);
-            } else if (i < n) {
+            } else {
                 // encoding gradient: columns 2 lv, 2 lv + 1 of dX_0
-                for (int lv = 0; lv < GUIDE_LEVELS; lv++) {
-                    const float gx = x[2 * lv], gy = x[2 * lv + 1];
-                    if (A.dbg_enc) {
-                        A.dbg_enc[(size_t)i * 32 + 2 * lv] = gx;
-                        A.dbg_enc[(size_t)i * 32 + 2 * lv + 1] = gy;
-                    }
-                    if (A.grid_grad) {
-                        Corners c;
-                        grid_corners(N, lv, p, c);
+                tc_load8(tmem + lane_addr + 8u * q, x);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                        for (int k = 0; k < 8; k++) {
-                            atomicAdd(&A.grid_grad[2 * (size_t)c.idx[k]], to_fixed(c.w[k] * gx));
-                            atomicAdd(&A.grid_grad[2 * (size_t)c.idx[k] + 1], to_fixed(c.w[k] * gy));
-                        }
+                for (int k = 0; k < GUIDE_LEVELS / 4; k++) {
+                    const int lv = k + (int)q * (GUIDE_LEVELS / 4);
+                    if (A.dbg_enc && live) {
+                        A.dbg_enc[(size_t)i * 32 + 2 * lv] = x[2 * k];
+                        A.dbg_enc[(size_t)i * 32 + 2 * lv + 1] = x[2 * k + 1];
                     }
+                    if (A.grid_grad) scatter_level(N, A.grid_grad, lv, p, live, x[2 * k], x[2 * k + 1]);
                 }
             }
         }
@@ -1152,20 +1201,26 @@ __global__ void __launch_bounds__(kTcRows, 1) k_guide_train_tc(GuideNetDev N, Tr
     if (!ok && tid == 0) tc_wait(mbar, phase);   // let a commit still in flight land
     __syncthreads();
     float *part = A.part + (size_t)blockIdx.x * kPart;
-    if (warp < 2) {
-        // dW_l[u][o] at tensor-memory lane u (0..63), column 64 (l + 1) + o
-        const uint32_t u = 32u * warp + lane;
-        for (int l = 0; l < GUIDE_LAYERS; l++) {
-            float v[W];
+    if ((warp & 3u) < 2) {
+        // dW_l[u][o] at tensor-memory lane u (0..63), column 64 (l + 1) + o; quarter l writes layer l
+        const uint32_t u = 32u * (warp & 3u) + lane;
+        float4 *dst = reinterpret_cast<float4 *>(part + (size_t)q * W * W + u * W);
 #pragma unroll
-            for (int c = 0; c < 4; c++) tc_load16(tmem + lane_addr + 64u * (uint32_t)(l + 1) + 16u * c, v + 16 * c);
+        for (int c = 0; c < 4; c++) {
+            float v[16];
+            tc_load16(tmem + lane_addr + 64u * (q + 1) + 16u * c, v);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            for (int o = 0; o < W; o++) part[(size_t)l * W * W + u * W + o] = has_acc && ok ? v[o] : 0.0f;
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                dst[4 * c + j] = has_acc && ok ? make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3])
+                                               : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
     }
+    if (q == 0) {
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) loss_acc += __shfl_down_sync(0xFFFFFFFFu, loss_acc, off);
-    if (lane == 0) s_loss[warp] = loss_acc;
+        for (int off = 16; off > 0; off >>= 1) loss_acc += __shfl_down_sync(0xFFFFFFFFu, loss_acc, off);
+        if (lane == 0) s_loss[warp] = loss_acc;
+    }
     __syncthreads();
     for (uint32_t j = tid; j < (uint32_t)W; j += blockDim.x) part[NW + j] = s_db[j];
     if (tid == 0) {
@@ -1196,14 +1251,46 @@ struct AdamStep {
     float lr, b1, b2, eps, c1, c2;   // c1, c2: bias corrections 1 / (1 - b^t)
 };
 
-__global__ void k_adam(float *w, float *g, float *m, float *v, uint32_t n, AdamStep a) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float gi = g[i];
-        g[i] = 0.0f;
-        const float mi = a.b1 * m[i] + (1.0f - a.b1) * gi, vi = a.b2 * v[i] + (1.0f - a.b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        w[i] -= a.lr * (mi * a.c1) / (sqrtf(vi * a.c2) + a.eps);
+__device__ __forceinline__ float adam(float *w, float *m, float *v, uint32_t i, float gi, const AdamStep &a) {
+    const float mi = a.b1 * m[i] + (1.0f - a.b1) * gi, vi = a.b2 * v[i] + (1.0f - a.b2) * gi * gi;
+    m[i] = mi;
+    v[i] = vi;
+    const float wi = w[i] - a.lr * (mi * a.c1) / (sqrtf(vi * a.c2) + a.eps);
+    w[i] = wi;
+    return wi;
+}
+
+// 16-bit position in a set of B fragments of the element in row k, column n of
+// layer l's B operand (k_frags).
+__device__ __forceinline__ uint32_t frag_at(uint32_t l, uint32_t k, uint32_t n) {
+    const uint32_t lane = (n & 7u) * 4u + ((k & 7u) >> 1);
+    return ((((l * 4u + (k >> 4)) * 8u + (n >> 3)) * 32u + lane) << 2) + ((k & 8u) >> 2) + (k & 1u);
+}
+
+// The end of a step for the dense parameters, a thread each: the blocks' slots
+// added up in block order, Adam, and the BF16 copies that the kernels read.
+// Five launches of a few microseconds each before (reduction, Adam for weights
+// and biases, the two sets of operands).
+__global__ void __launch_bounds__(128) k_guide_update(const float *part, uint32_t blocks, float *w, float *m, float *v,
+                                                      float *bias, float *bias_m, float *bias_v, float *loss, AdamStep a,
+                                                      __nv_bfloat16 *wtc, __nv_bfloat16 *wf, __nv_bfloat16 *wt) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i > (uint32_t)(NW + W)) return;
+    float s = 0.0f;
+#pragma unroll 16
+    for (uint32_t b = 0; b < blocks; b++) s += part[(size_t)b * kPart + i];
+    if (i == (uint32_t)(NW + W)) {
+        *loss = s;
+    } else if (i >= (uint32_t)NW) {
+        adam(bias, bias_m, bias_v, i - NW, s, a);
+    } else {
+        const __nv_bfloat16 x = __float2bfloat16_rn(adam(w, m, v, i, s, a));
+        const uint32_t l = i / (W * W), k = (i / W) % W, n = i % W;   // W[l][input unit k][output unit n]
+        unsigned char *base = reinterpret_cast<unsigned char *>(wtc) + (size_t)l * W * W * 2;
+        *reinterpret_cast<__nv_bfloat16 *>(base + tc_offset(n, k)) = x;
+        *reinterpret_cast<__nv_bfloat16 *>(base + (size_t)NW * 2 + tc_offset(k, n)) = x;
+        wf[frag_at(l, k, n)] = x;
+        wt[frag_at(l, n, k)] = x;
     }
 }
 
@@ -1374,7 +1461,9 @@ constexpr float kWeightCap = 25.0f;
 
 // One training step over rows[0 .. min(*count, cap)): gradients, then Adam.
 int TrainStep(GuideState &g, const GuideRow *rows, const uint32_t *count, uint32_t cap, const float *wsum,
-              cudaStream_t st, float *dbg_out = nullptr, float *dbg_enc = nullptr, bool apply = true) {
+              cudaStream_t st, float *dbg_out = nullptr, float *dbg_enc = nullptr, bool apply = true,
+              float *loss = nullptr) {
+    if (!loss) loss = g.loss;
     TrainArgs A;
     A.rows = rows;
     A.count = count;
@@ -1385,11 +1474,14 @@ int TrainStep(GuideState &g, const GuideRow *rows, const uint32_t *count, uint32
     A.grid_grad = g.grid_grad;
     A.dbg_out = dbg_out;
     A.dbg_enc = dbg_enc;
-    if (g.use_tc) k_guide_train_tc<<<g.sms, kTcRows, kTcTrainSmem, st>>>(g.net, A, g.tc_error);
+    if (g.use_tc) k_guide_train_tc<<<g.sms, kTcTrainThreads, kTcTrainSmem, st>>>(g.net, A, g.tc_error);
     else k_guide_train<<<g.sms, kWarps * 32, kTrainSmem, st>>>(g.net, A);
-    k_guide_reduce<<<(NW + W + 1 + 255) / 256, 256, 0, st>>>(g.part, (uint32_t)g.sms, g.w_grad, g.b_grad, g.loss);
     AZ_CUDA_TRY(cudaGetLastError());
-    if (!apply) return AZ_OK;
+    if (!apply) {
+        k_guide_reduce<<<(NW + W + 1 + 255) / 256, 256, 0, st>>>(g.part, (uint32_t)g.sms, g.w_grad, g.b_grad, loss);
+        AZ_CUDA_TRY(cudaGetLastError());
+        return AZ_OK;
+    }
     g.step++;
     AdamStep a;
     a.lr = g.lr;
@@ -1398,11 +1490,12 @@ int TrainStep(GuideState &g, const GuideRow *rows, const uint32_t *count, uint32
     a.eps = 1e-8f;
     a.c1 = (float)(1.0 / (1.0 - std::pow(0.9, (double)g.step)));
     a.c2 = (float)(1.0 / (1.0 - std::pow(0.99, (double)g.step)));
-    k_adam<<<16, 256, 0, st>>>(g.w, g.w_grad, g.w_m, g.w_v, NW, a);
-    k_adam<<<1, 64, 0, st>>>(g.bias, g.b_grad, g.b_m, g.b_v, W, a);
+    k_guide_update<<<(NW + W + 1 + 127) / 128, 128, 0, st>>>(
+        g.part, (uint32_t)g.sms, g.w, g.w_m, g.w_v, g.bias, g.b_m, g.b_v, loss, a, g.wtc,
+        reinterpret_cast<__nv_bfloat16 *>(g.wf), reinterpret_cast<__nv_bfloat16 *>(g.wt));
     k_adam_grid<<<g.sms * 8, 256, 0, st>>>(g.grid, g.grid_grad, g.grid_m, g.grid_v, g.feat, kGridN, a);
     AZ_CUDA_TRY(cudaGetLastError());
-    return RefreshFragments(g, st);
+    return AZ_OK;
 }
 
 }  // namespace
@@ -1818,27 +1911,36 @@ extern "C" int az_guide_eval(az_guide *g, const float *rows, uint32_t n, float *
     return rc;
 }
 
+// The rows and the steps' losses are in pool memory and the losses come back
+// together: an allocation of 6 MB and its release took 0.8 ms, as long as two
+// steps on 100,003 rows.
+static int TrainRows(GuideState &s, const float *rows, uint32_t n, uint32_t steps, float *losses, cudaStream_t st) {
+    PoolBuf<GuideRow> d_rows;
+    PoolBuf<uint32_t> d_count;
+    PoolBuf<float> d_loss;
+    AZ_CUDA_TRY(d_rows.alloc(n, st));
+    AZ_CUDA_TRY(d_count.alloc(1, st));
+    AZ_CUDA_TRY(d_loss.alloc(steps, st));
+    AZ_CUDA_TRY(cudaMemcpyAsync(d_rows.p, rows, (size_t)n * sizeof(GuideRow), cudaMemcpyHostToDevice, st));
+    AZ_CUDA_TRY(cudaMemcpyAsync(d_count.p, &n, sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+    int rc = AZ_OK;
+    for (uint32_t k = 0; k < steps && rc == AZ_OK; k++)
+        rc = TrainStep(s, d_rows.p, d_count.p, n, nullptr, st, nullptr, nullptr, true, d_loss.p + k);
+    if (rc != AZ_OK) return rc;
+    if (losses && steps)
+        AZ_CUDA_TRY(cudaMemcpyAsync(losses, d_loss.p, steps * sizeof(float), cudaMemcpyDeviceToHost, st));
+    return GuideCheck(s, st);   // waits for the steps
+}
+
 extern "C" int az_guide_train(az_guide *g, const float *rows, uint32_t n, uint32_t steps, float *losses) {
     if (!g || (n && !rows)) return SetError(AZ_ERR_INVALID_ARGUMENT, "null argument");
     GuideState &s = *g->impl;
     AZ_CUDA_TRY(cudaSetDevice(s.device));
-    GuideRow *d_rows = nullptr;
-    uint32_t *d_count = nullptr;
-    int rc = UploadRows(s, rows, n, &d_rows, &d_count);
-    for (uint32_t k = 0; k < steps && rc == AZ_OK; k++) {
-        rc = TrainStep(s, d_rows, d_count, n, nullptr, nullptr);
-        if (rc == AZ_OK && losses) {
-            cudaError_t e = cudaMemcpy(&losses[k], s.loss, sizeof(float), cudaMemcpyDeviceToHost);
-            if (e != cudaSuccess) rc = CudaError(e, "guide train");
-        }
-    }
-    if (rc == AZ_OK) {
-        cudaError_t e = cudaDeviceSynchronize();
-        if (e != cudaSuccess) rc = CudaError(e, "guide train");
-    }
-    if (rc == AZ_OK) rc = GuideCheck(s, nullptr);
-    cudaFree(d_rows);
-    cudaFree(d_count);
+    // a blocking stream: after earlier work on the legacy default stream
+    cudaStream_t st = nullptr;
+    AZ_CUDA_TRY(AcquireStream(&st));
+    const int rc = TrainRows(s, rows, n, steps, losses, st);
+    ReleaseStream(st);
     return rc;
 }
 
