@@ -64,7 +64,6 @@ __device__ __forceinline__ void camera_node(const CameraParams &cam, const WaveQ
     Q.o[1][i] = make_float4(o.x, o.y, o.z, time);
     Q.d[1][i] = make_float4(dir.x, dir.y, dir.z, __uint_as_float(cam.scene << PF_SCENE_SHIFT));
     Q.tp[1][i] = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(i));
-    Q.att[1][i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     Q.digits[1][i] = 0u;
     Q.accum[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 }
@@ -578,6 +577,9 @@ int SetupCamera(const az_camera *c, az_scissor sc, int32_t filter, uint32_t cull
     cam.hsc = r1 > cam.r0 ? r1 - cam.r0 : 0;
     cam.wsc = c1 > cam.c0 ? c1 - cam.c0 : 0;
     cam.npix = (uint64_t)cam.hsc * cam.wsc;
+    cam.by_npix.set((uint32_t)cam.npix);   // at most 65535^2
+    cam.by_wsc.set(cam.wsc);
+    cam.by_sqrt.set(cam.sqrt_spp);
     if (filter != AZ_Filter_Box && filter != AZ_Filter_Gaussian) return SetError(AZ_ERR_INVALID_ARGUMENT, "unknown filter");
     cam.filter = filter;
     cam.seed = seed;

@@ -25,12 +25,32 @@ constexpr uint32_t AZ_COUNT_TOTAL = 4 * AZ_MAX_LEVELS + 8;
 
 // Camera and film parameters of one render call (ProduceImageInLinearSpace's
 // locals, src/azimuth_main.cpp:1265-1347).
+// Division of 32-bit numbers by a number that a launch keeps (Granlund,
+// Montgomery, "Division by Invariant Integers using Multiplication", PLDI
+// 1994): the quotient from a 64-bit product, for every dividend.
+struct FastDiv {
+    uint32_t d, m, sh1, sh2;
+    void set(uint32_t divisor) {
+        d = divisor ? divisor : 1u;
+        uint32_t l = 0;
+        while (l < 32 && ((uint64_t)1 << l) < d) l++;   // ceil(log2 d)
+        m = (uint32_t)((((uint64_t)1 << 32) * (((uint64_t)1 << l) - d)) / d + 1u);
+        sh1 = l < 1 ? l : 1u;
+        sh2 = l < 1 ? 0u : l - 1u;
+    }
+    __host__ __device__ __forceinline__ uint32_t quotient(uint32_t n) const {
+        const uint32_t t = (uint32_t)(((uint64_t)m * n) >> 32);
+        return (t + ((n - t) >> sh1)) >> sh2;
+    }
+};
+
 struct CameraParams {
     azd::f3 base, pos, axx, axy, stepx, stepy;
     float aperture, inv_sqrt;
     uint32_t sqrt_spp, width, height;
     uint32_t r0, c0, wsc, hsc;     // scissor origin and size
     uint64_t npix;
+    FastDiv by_npix, by_wsc, by_sqrt;   // npix (below 2^32), wsc, sqrt_spp
     int32_t filter;
     float g_norm, g_neg;
     int32_t gk;

@@ -34,13 +34,23 @@ __host__ __device__ __forceinline__ uint32_t shadow_light(uint32_t meta) { retur
 // Most scenes a tile wave can hold (the 8-bit scene index above)
 constexpr uint32_t kMaxWaveScenes = 256;
 
+// Every shaded node asks for its sample's pixel.  Three 64-bit divisions were
+// about a sixth of a node's instructions; samples beyond 2^32 still take one.
 __host__ __device__ __forceinline__ void sample_of(const CameraParams &cam, uint64_t s, uint32_t &row,
                                                    uint32_t &col, uint32_t &sx, uint32_t &sy) {
-    uint64_t pix = s % cam.npix, k = s / cam.npix;
-    row = cam.r0 + (uint32_t)(pix / cam.wsc);
-    col = cam.c0 + (uint32_t)(pix % cam.wsc);
-    sx = (uint32_t)(k % cam.sqrt_spp);
-    sy = (uint32_t)(k / cam.sqrt_spp);
+    uint32_t pix, k;
+    if (s >> 32) {
+        k = (uint32_t)(s / cam.npix);
+        pix = (uint32_t)(s % cam.npix);
+    } else {
+        k = cam.by_npix.quotient((uint32_t)s);
+        pix = (uint32_t)s - k * cam.by_npix.d;
+    }
+    const uint32_t y = cam.by_wsc.quotient(pix);
+    row = cam.r0 + y;
+    col = cam.c0 + (pix - y * cam.by_wsc.d);
+    sy = cam.by_sqrt.quotient(k);
+    sx = k - sy * cam.by_sqrt.d;
 }
 
 __device__ __forceinline__ uint32_t push_slot(uint32_t *counter) {
@@ -70,7 +80,7 @@ __device__ __forceinline__ void push_path(const WaveQueues &Q, int buf, uint32_t
     Q.o[buf][i] = make_float4(o.x, o.y, o.z, time);
     Q.d[buf][i] = make_float4(d.x, d.y, d.z, __uint_as_float(flags));
     Q.tp[buf][i] = make_float4(tp.x, tp.y, tp.z, __uint_as_float(slot));
-    Q.att[buf][i] = make_float4(att.x, att.y, att.z, 0.0f);
+    if (flags & PF_ATTEN) Q.att[buf][i] = make_float4(att.x, att.y, att.z, 0.0f);   // read for these only
     Q.digits[buf][i] = digits;
 }
 
