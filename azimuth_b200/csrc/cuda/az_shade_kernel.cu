@@ -22,8 +22,14 @@ __device__ __forceinline__ f3 ld3(const float *p) { return mk(p[0], p[1], p[2]);
 // branches, point/area/directional/spot lights.  MULTI: a tile wave of
 // several scenes, each entry shaded in the scene its flags name (FEAT then
 // covers every scene of the wave).
+//
+// Bound by latency (long dependent chains on few warps: 28 % of the SM's warps
+// with the 92-96 registers the compiler takes).  Eight blocks of 64 registers an
+// SM win although they spill: features scene of 3.8 M samples 45.3 -> 40.2 ms a
+// frame (six blocks: 43.7), 24 tile jobs of three scenes 28.1 -> 26.3, dense mesh
+// 199.6 -> 196.1.
 template <int BLOCK, uint32_t FEAT, bool GUIDED, bool TILES = false, bool MULTI = false>
-__global__ void __launch_bounds__(BLOCK) k_shade(DevScene S0, CameraParams cam, WaveQueues Q, uint64_t wave_start,
+__global__ void __launch_bounds__(BLOCK, 8) k_shade(DevScene S0, CameraParams cam, WaveQueues Q, uint64_t wave_start,
                                                  uint32_t level) {
     constexpr bool TEX = FEAT & FEAT_TEXTURES, ENV = FEAT & FEAT_ENV, SPECIAL = FEAT & FEAT_SPECIAL,
                    LIGHTS = FEAT & FEAT_ANALYTIC_LIGHTS;
