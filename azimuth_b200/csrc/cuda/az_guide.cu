@@ -112,15 +112,28 @@ __device__ __forceinline__ void grid_corners(const GuideNetDev &N, int l, f3 p, 
     }
 }
 
+// The gathers are bound by the entries a warp touches.  Corners 2j and 2j + 1
+// are neighbours in x: in half of all cells (even x in a hashed level, even
+// index in a dense one) their entries share an aligned pair, and one 8-byte
+// load brings both.
 __device__ __forceinline__ float2 grid_feature(const GuideNetDev &N, int l, f3 p) {
     Corners c;
     grid_corners(N, l, p, c);
+    const uint2 *pairs = reinterpret_cast<const uint2 *>(N.grid);
+    uint32_t v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k += 2) {
+        const uint2 u = __ldg(pairs + (c.idx[k] >> 1));
+        v[k] = c.idx[k] & 1u ? u.y : u.x;
+        v[k + 1] = c.idx[k] & 1u ? u.x : u.y;
+        if ((c.idx[k] ^ c.idx[k + 1]) != 1u) v[k + 1] = __ldg(reinterpret_cast<const uint32_t *>(N.grid) + c.idx[k + 1]);
+    }
     float2 f = make_float2(0.0f, 0.0f);
 #pragma unroll
     for (int k = 0; k < 8; k++) {
-        const float2 v = __half22float2(N.grid[c.idx[k]]);
-        f.x += c.w[k] * v.x;
-        f.y += c.w[k] * v.y;
+        const float2 e = __half22float2(*reinterpret_cast<const __half2 *>(&v[k]));
+        f.x += c.w[k] * e.x;
+        f.y += c.w[k] * e.y;
     }
     return f;
 }
@@ -1399,6 +1412,7 @@ struct GuideState {
     uint32_t *row_keys = nullptr, *row_order = nullptr;   // [row_cap] (OrderRows)
     uint32_t row_cap = 0;
     uint32_t *bin_counts = nullptr, *bin_offsets = nullptr;
+    uint32_t *bin_block_base = nullptr;                   // [sms * 4][kSortBins]
     unsigned char *bin_scan_temp = nullptr;
     size_t bin_scan_bytes = 0;
     std::mutex mu;
@@ -1657,35 +1671,50 @@ __device__ __forceinline__ uint32_t row_bin(const WaveQueues &Q, int buf, uint32
     return (spread4(x) << 2) | (spread4(y) << 1) | spread4(z);
 }
 
-// PASS 0: count rows per bin (keys kept); PASS 1: place every row at its bin's
-// next slot.  Loop bounds are warp-uniform so that lanes with equal keys can
-// share one atomic.
-template <int PASS>
-__global__ void k_guide_bins(WaveQueues Q, uint32_t level, GuideNetDev N, uint32_t *keys, uint32_t *bins,
-                             uint32_t *order) {
+// A block counts a run of rows in shared memory and takes its part of each bin
+// with one atomic; a row's rank within the block's part stays with its key, so
+// the second pass needs no atomics (20 M rows of a guided 1280x720 pass: two
+// passes with an atomic per warp and bin took 1.58 ms).
+constexpr uint32_t kBinBlock = 512;
+constexpr uint32_t kBinRankShift = 12;   // key in the low bits: a block's run is below 2^20 rows
+
+// The block's run of rows: [first, last), a multiple of 32 rows long.
+__device__ __forceinline__ void bin_run(uint32_t n, uint32_t &first, uint32_t &last) {
+    const uint32_t run = ((n + gridDim.x - 1) / gridDim.x + 31u) & ~31u;
+    first = min(n, blockIdx.x * run);
+    last = min(n, first + run);
+}
+
+__global__ void __launch_bounds__(kBinBlock) k_guide_bin_count(WaveQueues Q, uint32_t level, GuideNetDev N,
+                                                               uint32_t *keys, uint32_t *bins, uint32_t *block_base) {
+    __shared__ uint32_t count[kSortBins];
     const uint32_t n = min(Q.counts[level], Q.cap_q);
     const int buf = level & 1;
-    const uint32_t lane = threadIdx.x & 31u;
-    for (uint32_t b = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); b < n; b += gridDim.x * blockDim.x) {
-        const uint32_t i = b + lane;
-        const bool live = i < n;
-        uint32_t key = 0xFFFFFFFFu;
-        if (live) {
-            if (PASS == 0) {
-                key = row_bin(Q, buf, i, N);
-                keys[i] = key;
-            } else {
-                key = keys[i];
-            }
-        }
-        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, key);
-        const uint32_t leader = __ffs(peers) - 1u;
-        uint32_t base = 0;
-        if (live && lane == leader) base = atomicAdd(&bins[key], (uint32_t)__popc(peers));
-        if (PASS == 1) {
-            base = __shfl_sync(0xFFFFFFFFu, base, leader);
-            if (live) order[base + __popc(peers & ((1u << lane) - 1u))] = i;
-        }
+    uint32_t first, last;
+    bin_run(n, first, last);
+    if (first == last) return;
+    for (uint32_t b = threadIdx.x; b < kSortBins; b += kBinBlock) count[b] = 0u;
+    __syncthreads();
+    for (uint32_t i = first + threadIdx.x; i < last; i += kBinBlock) {
+        const uint32_t key = row_bin(Q, buf, i, N);
+        keys[i] = key | (atomicAdd(&count[key], 1u) << kBinRankShift);
+    }
+    __syncthreads();
+    for (uint32_t b = threadIdx.x; b < kSortBins; b += kBinBlock)
+        if (count[b]) block_base[blockIdx.x * kSortBins + b] = atomicAdd(&bins[b], count[b]);
+}
+
+// Every row to its bin's first slot + its block's part + its rank there.
+__global__ void __launch_bounds__(kBinBlock) k_guide_bin_place(WaveQueues Q, uint32_t level, const uint32_t *keys,
+                                                               const uint32_t *offsets, const uint32_t *block_base,
+                                                               uint32_t *order) {
+    const uint32_t n = min(Q.counts[level], Q.cap_q);
+    uint32_t first, last;
+    bin_run(n, first, last);
+#pragma unroll 4
+    for (uint32_t i = first + threadIdx.x; i < last; i += kBinBlock) {
+        const uint32_t k = keys[i], key = k & (kSortBins - 1u);
+        order[__ldg(offsets + key) + __ldg(block_base + blockIdx.x * kSortBins + key) + (k >> kBinRankShift)] = i;
     }
 }
 
@@ -1694,7 +1723,7 @@ static int OrderRows(GuideState &g, const WaveQueues &Q, uint32_t level, cudaStr
 int GuideInfer(GuideState &g, const GpuScene &G, const WaveQueues &Q, uint32_t level, cudaStream_t st) {
     if (g.use_tc) {
         const uint32_t *order = nullptr;
-        if (g.order_rows) {
+        if (g.order_rows && Q.cap_q / ((uint32_t)g.sms * 4) < (1u << (32 - kBinRankShift)) - 32u) {
             int rc = OrderRows(g, Q, level, st);
             if (rc != AZ_OK) return rc;
             order = g.row_order;
@@ -1725,15 +1754,17 @@ static int OrderRows(GuideState &g, const WaveQueues &Q, uint32_t level, cudaStr
         g.bin_scan_bytes = bytes;
         g.bin_counts = g.Alloc<uint32_t>(kSortBins);
         g.bin_offsets = g.Alloc<uint32_t>(kSortBins);
+        g.bin_block_base = g.Alloc<uint32_t>((size_t)g.sms * 4 * kSortBins);
         g.bin_scan_temp = g.Alloc<unsigned char>(std::max<size_t>(bytes, 16));
-        if (!g.bin_counts || !g.bin_offsets || !g.bin_scan_temp) return SetError(AZ_ERR_OUT_OF_MEMORY, "row bins");
+        if (!g.bin_counts || !g.bin_offsets || !g.bin_block_base || !g.bin_scan_temp)
+            return SetError(AZ_ERR_OUT_OF_MEMORY, "row bins");
     }
     AZ_CUDA_TRY(cudaMemsetAsync(g.bin_counts, 0, kSortBins * sizeof(uint32_t), st));
-    const int grid = g.sms * 8;
-    k_guide_bins<0><<<grid, 256, 0, st>>>(Q, level, g.net, g.row_keys, g.bin_counts, nullptr);
+    k_guide_bin_count<<<g.sms * 4, kBinBlock, 0, st>>>(Q, level, g.net, g.row_keys, g.bin_counts, g.bin_block_base);
     size_t bytes = g.bin_scan_bytes;
     AZ_CUDA_TRY(cub::DeviceScan::ExclusiveSum(g.bin_scan_temp, bytes, g.bin_counts, g.bin_offsets, (int)kSortBins, st));
-    k_guide_bins<1><<<grid, 256, 0, st>>>(Q, level, g.net, g.row_keys, g.bin_offsets, g.row_order);
+    k_guide_bin_place<<<g.sms * 4, kBinBlock, 0, st>>>(Q, level, g.row_keys, g.bin_offsets, g.bin_block_base,
+                                                          g.row_order);
     AZ_CUDA_TRY(cudaGetLastError());
     return AZ_OK;
 }
