@@ -13,6 +13,7 @@ struct DevicePools {
     std::mutex mu;
     cudaMemPool_t pool[kMaxDevices] = {};
     std::vector<cudaStream_t> streams[kMaxDevices];
+    std::vector<SideStream> sides[kMaxDevices];
     cudaStream_t idle[kMaxDevices] = {};   // takes the frees of memory that no work uses any more
     std::unordered_set<void *> direct;     // buffers of cudaMalloc
 };
@@ -140,6 +141,47 @@ void ReleaseStream(cudaStream_t st) {
         }
     }
     cudaStreamDestroy(st);
+}
+
+cudaError_t AcquireSide(SideStream *s) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev >= 0 && dev < kMaxDevices) {
+        DevicePools &P = Pools();
+        std::lock_guard<std::mutex> lock(P.mu);
+        if (!P.sides[dev].empty()) {
+            *s = P.sides[dev].back();
+            P.sides[dev].pop_back();
+            return cudaSuccess;
+        }
+    }
+    SideStream n;
+    e = cudaStreamCreateWithFlags(&n.stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&n.fork, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&n.join, cudaEventDisableTiming);
+    if (e != cudaSuccess) {
+        if (n.fork) cudaEventDestroy(n.fork);
+        if (n.stream) cudaStreamDestroy(n.stream);
+        return e;
+    }
+    *s = n;
+    return cudaSuccess;
+}
+
+void ReleaseSide(const SideStream &s) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices) {
+        DevicePools &P = Pools();
+        std::lock_guard<std::mutex> lock(P.mu);
+        if (P.sides[dev].size() < kStreamsKept) {
+            P.sides[dev].push_back(s);
+            return;
+        }
+    }
+    cudaEventDestroy(s.fork);
+    cudaEventDestroy(s.join);
+    cudaStreamDestroy(s.stream);
 }
 
 }  // namespace az

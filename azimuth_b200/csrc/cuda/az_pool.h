@@ -51,4 +51,14 @@ constexpr size_t kStreamsKept = 8;
 cudaError_t AcquireStream(cudaStream_t *st);
 void ReleaseStream(cudaStream_t st);
 
+// A non-blocking stream with the two events that order it against a render's
+// stream (it only ever runs after waiting on `fork`); idle ones are kept as above.
+// ReleaseSide: when nothing runs on it any more.
+struct SideStream {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+};
+cudaError_t AcquireSide(SideStream *s);
+void ReleaseSide(const SideStream &s);
+
 }  // namespace az

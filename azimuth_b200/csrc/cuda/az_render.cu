@@ -593,33 +593,21 @@ WaveBuffers::~WaveBuffers() {
     DropGraph();
     // every render waits for its waves, so nothing uses the buffers any more
     for (void *p : ptrs) PoolFree(p, nullptr);
-    if (wave_host) cudaFreeHost(wave_host);
     PoolFree(guide_lobes, nullptr);
     PoolFree(guide_rec, nullptr);
     for (void *p : {(void *)okey[0], (void *)okey[1], (void *)oval, (void *)oidx_e, (void *)oidx_s, otemp})
         PoolFree(p, nullptr);
-    if (ev_fork) cudaEventDestroy(ev_fork);
-    if (ev_join) cudaEventDestroy(ev_join);
-    if (side) cudaStreamDestroy(side);
+    if (side) ReleaseSide(SideStream{side, ev_fork, ev_join});
 }
 
 int WaveBuffers::EnsureSide() {
     if (side) return AZ_OK;
-    // non-blocking: the side stream only ever runs after waiting on an event
-    // of the render stream, which orders it after the caller's earlier work
-    cudaStream_t s = nullptr;
-    cudaEvent_t f = nullptr, j = nullptr;
-    cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&f, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&j, cudaEventDisableTiming);
-    if (e != cudaSuccess) {
-        if (f) cudaEventDestroy(f);
-        if (s) cudaStreamDestroy(s);
-        return CudaError(e, "creating the wave's side stream");
-    }
-    side = s;
-    ev_fork = f;
-    ev_join = j;
+    SideStream s;
+    const cudaError_t e = AcquireSide(&s);
+    if (e != cudaSuccess) return CudaError(e, "creating the wave's side stream");
+    side = s.stream;
+    ev_fork = s.fork;
+    ev_join = s.join;
     return AZ_OK;
 }
 
@@ -680,10 +668,6 @@ int WaveBuffers::Ensure(uint32_t chunk, uint32_t cap_q, uint32_t cap_s, cudaStre
     wave_dev = (uint64_t *)alloc(4 * sizeof(uint64_t));
     if (!q.hit || !q.so || !q.sd || !q.sc || !q.smeta || !q.accum || !q.counts || !wave_dev)
         return SetError(AZ_ERR_OUT_OF_MEMORY, "wave queues");
-    if (!wave_host && cudaMallocHost((void **)&wave_host, 4 * sizeof(uint64_t)) != cudaSuccess) {
-        wave_host = nullptr;
-        return SetError(AZ_ERR_OUT_OF_MEMORY, "wave descriptor");
-    }
     q.cap_q = cap_q;
     q.cap_s = cap_s;
     this->chunk = chunk;
@@ -851,8 +835,16 @@ static int RenderWave(const GpuScene &G, const CameraParams &cam, WaveBuffers &W
     return AZ_OK;
 }
 
-// One wave through the captured graph of W (capturing it first when the
-// scene, camera, film, launch configuration or largest wave changed).
+// The descriptor that a replayed wave reads (no pinned memory to keep, and no
+// wait for a copy from pageable memory).
+__global__ void k_set_wave(uint64_t *wave, uint64_t start, uint64_t n, uint64_t seed) {
+    wave[0] = start;
+    wave[1] = n;
+    wave[2] = seed;
+}
+
+// One wave through the captured graph of W (captured on the second wave of the
+// same scene, camera, film, launch configuration and largest wave).
 static int ReplayWave(const GpuScene &G, const CameraParams &cam, WaveBuffers &W, uint64_t start, uint32_t n,
                       uint32_t n_max, az_pixel *film, cudaStream_t st, int sms, RenderCounters &rc) {
     struct Key {
@@ -875,7 +867,17 @@ static int ReplayWave(const GpuScene &G, const CameraParams &cam, WaveBuffers &W
     key.q0 = W.q.o[0];
     const unsigned char *kb = reinterpret_cast<const unsigned char *>(&key);
     RenderCounters launches{};
-    if (!W.graph || W.graph_key.size() != sizeof(key) || memcmp(W.graph_key.data(), kb, sizeof(key)) != 0) {
+    const auto same = [&](const std::vector<unsigned char> &k) {
+        return k.size() == sizeof(key) && memcmp(k.data(), kb, sizeof(key)) == 0;
+    };
+    if (!W.graph || !same(W.graph_key)) {
+        // The first wave of a kind is launched directly: capturing and
+        // instantiating its graph takes as long as several waves of a small
+        // render, and a one-shot image has no second one.
+        if (!same(W.direct_key)) {
+            W.direct_key.assign(kb, kb + sizeof(key));
+            return RenderWave(G, cam, W, start, n, film, st, sms, rc, nullptr, nullptr, false);
+        }
         W.DropGraph();
         AZ_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
         int crc = RenderWave(G, cam, W, 0, n_max, film, st, sms, launches, nullptr, nullptr, false, true);
@@ -896,10 +898,7 @@ static int ReplayWave(const GpuScene &G, const CameraParams &cam, WaveBuffers &W
         W.graph_launches = launches.launches;
         W.graph_extend_launches = launches.extend_launches;
     }
-    W.wave_host[0] = start;
-    W.wave_host[1] = n;
-    W.wave_host[2] = cam.seed;
-    AZ_CUDA_TRY(cudaMemcpyAsync(W.wave_dev, W.wave_host, 3 * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
+    k_set_wave<<<1, 1, 0, st>>>(W.wave_dev, start, n, cam.seed);
     AZ_CUDA_TRY(cudaGraphLaunch(W.graph, st));
     rc.launches += W.graph_launches;
     rc.extend_launches += W.graph_extend_launches;

@@ -120,9 +120,9 @@ struct WaveBuffers {
     std::vector<void *> ptrs;
     // the per-wave launches captured as a CUDA graph, with what they were captured for
     uint64_t *wave_dev = nullptr;          // device copy of the wave descriptor
-    uint64_t *wave_host = nullptr;         // pinned staging for it
     cudaGraphExec_t graph = nullptr;
     std::vector<unsigned char> graph_key;
+    std::vector<unsigned char> direct_key;   // of the last wave launched without a graph
     uint64_t graph_launches = 0, graph_extend_launches = 0;   // kernels in the graph
     // scratch of guided waves: proposals per queue entry, training records
     azd::GuideLobes *guide_lobes = nullptr;
@@ -138,7 +138,7 @@ struct WaveBuffers {
     // second stream of a wave: a level's visibility queries run on it beside
     // the next level's closest-hit queries (fork after shading, join before
     // the next shading)
-    cudaStream_t side = nullptr;
+    cudaStream_t side = nullptr;          // SideStream
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     ~WaveBuffers();
     int EnsureSide();
