@@ -1016,9 +1016,9 @@ int Render(GpuScene &G, az_pixel *film, const az_camera *camera, const az_epsilo
     std::vector<uint32_t> host_counts(AZ_COUNT_TOTAL);
     std::unique_ptr<StageTimer> timer;
     if (stats && opts && (opts->flags & AZ_FLAG_TIME_STAGES)) timer.reset(new StageTimer());
-    // The launches of a wave run as one CUDA graph, captured once per scene,
-    // camera, film and launch configuration and replayed for every wave with
-    // its first sample, size and seed in a 24-byte descriptor.  Not for stage
+    // The launches of a wave run as one CUDA graph from the second wave of a
+    // scene, camera, film and launch configuration on (ReplayWave), with each
+    // wave's first sample, size and seed in a 24-byte descriptor.  Not for stage
     // timing, guided renders, or a legacy default stream (which cannot be
     // captured).
     const bool use_graph = !(opts && (opts->flags & AZ_FLAG_NO_GRAPH)) && !timer && !guide && st != nullptr &&

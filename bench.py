@@ -44,10 +44,10 @@ SCENE_ARGS = dict(scene_id=1, seed=0)
 # of every k_extend / k_shadow launch of one 256x256, 16-spp frame (one wave of
 # 2^20 samples): the capture's bytes over the frame's queries
 DRAM_BYTES_PER_QUERY = {"k_extend": 207.1, "k_shadow": 246.2}
-PROFILE_NOTE = "profiles/traversal_dram_dense_mesh_256x256_16spp.md, profiles/k_extend_k_shadow_dense_mesh_256x256_16spp.md"
+PROFILE_NOTE = "profiles/traversal_dram_dense_mesh_256x256_16spp.md, profiles/phase_traversal_dense_mesh_256x256_16spp.md"
 # issue statistics of the two traversal kernels from the ncu capture of that small case
-ISSUE = {"k_extend": {"threads_per_warp_instruction": 8.63, "issue_active_pct": 57.1, "warps_active_pct": 36.2},
-         "k_shadow": {"threads_per_warp_instruction": 8.47, "issue_active_pct": 56.2, "warps_active_pct": 34.3}}
+ISSUE = {"k_extend": {"threads_per_warp_instruction": 16.76, "issue_active_pct": 58.3, "warps_active_pct": 41.6},
+         "k_shadow": {"threads_per_warp_instruction": 16.91, "issue_active_pct": 52.3, "warps_active_pct": 41.3}}
 
 
 def parse():
@@ -358,7 +358,7 @@ def main():
                    if dense and DRAM_BYTES_PER_QUERY["k_extend"] else None)
     sh_traffic = (DRAM_BYTES_PER_QUERY["k_shadow"] * sh_q / launches_per_frame
                   if dense and DRAM_BYTES_PER_QUERY["k_shadow"] else None)
-    limiter = ("instruction issue of divergent traversal, not HBM: about 8 of 32 lanes active per warp "
+    limiter = ("instruction issue of divergent traversal, not HBM: about 17 of 32 lanes active per warp "
                "instruction, DRAM traffic a quarter of the algorithmic bytes (%s)" % PROFILE_NOTE)
     roofline = {"bound": "hbm", "achieved": ext_achieved, "peak": hbm, "unit": "GB/s", "frac": ext_achieved / hbm,
                 "traffic": ext_traffic, "traffic_unit": "DRAM bytes per launch (ncu, scaled from a small frame)",
