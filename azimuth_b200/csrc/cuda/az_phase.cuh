@@ -216,10 +216,8 @@ struct PhaseTracer {
         } else if (g.identity) {
             set_ray(local_ray_identity(wr));
             if (wlim < FLT_MAX) {
-                tcur = wlim * 1.0001f + 1e-30f;
-                // hits from here on are out of a visibility query's range (the local
-                // direction is a unit vector, the world one need not be)
-                if (KIND == Q_ANY) bl_t = wlim * length(wr.d) * 1.0001f + 1e-30f;
+                tcur = wlim * group_t_scale(g, wr.d) + 1e-30f;
+                if (KIND == Q_ANY) bl_t = tcur;   // hits from here on are out of a visibility query's range
             }
         } else {
             const GroupRay gr = group_ray_call(S.groups + gi, wr);

@@ -340,12 +340,11 @@ __device__ __forceinline__ float group_world_t(const DevGroup &g, const Ray &wr,
     return length(wp - o2 - motion) / length(wr.d);
 }
 
-// Factor from a world distance along d to the group's local distance
-// (|inv * d| / |d|) with a margin of 1e-4 for rounding; exactly 1.0001 for an
-// identity group, whose vector transform returns d unchanged.
+// Factor from a world distance, in units of d, to the group's local one, whose
+// direction is re-normalised: |inv * d|, with a margin of 1e-4 for rounding.  An
+// identity group's vector transform returns d unchanged.
 __device__ __forceinline__ float group_t_scale(const DevGroup &g, f3 d) {
-    if (g.identity) return 1.0001f;
-    return length(vector_xf(g.inv, d)) / length(d) * 1.0001f;
+    return length(g.identity ? d : vector_xf(g.inv, d)) * 1.0001f;
 }
 
 // sphere_test of entity e for the world ray.
@@ -562,7 +561,7 @@ __device__ bool trace(const DevScene &S, const Ray &wr, bool cull, float eps, fl
                 if (wlim < FLT_MAX) tcur = wlim + 1e-30f;
             } else if (g.identity) {
                 r = local_ray_identity(wr);
-                if (wlim < FLT_MAX) tcur = wlim * 1.0001f + 1e-30f;
+                if (wlim < FLT_MAX) tcur = wlim * group_t_scale(g, wr.d) + 1e-30f;
             } else {
                 const GroupRay gr = group_ray_call(S.groups + g_idx, wr);
                 r = gr.r;
