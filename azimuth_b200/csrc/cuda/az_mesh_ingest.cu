@@ -381,21 +381,26 @@ int SoupArea(const SoupWork &w, uint32_t mesh, float &area, cudaStream_t st) {
     return AZ_OK;
 }
 
+// IngestSoup does not wait for its kernels, and `st` may be a caller's non-blocking
+// stream: every copy is queued on it, and the call ends with a wait.
 int SoupRecords(const SoupWork &w, az_triangle *tris, az_face_attr *attrs, az_vec3 *vertex_normals,
                 cudaStream_t st) {
-    if (vertex_normals && w.nv)
-        AZ_CUDA_TRY(cudaMemcpy(vertex_normals, w.vn.p, (size_t)w.nv * 12, cudaMemcpyDeviceToHost));
-    if ((!tris && !attrs) || w.nf == 0) return AZ_OK;
     PoolBuf<az_triangle> dt;
     PoolBuf<az_face_attr> da;
-    if (tris) AZ_CUDA_TRY(dt.alloc(w.nf, st));
-    if (attrs) AZ_CUDA_TRY(da.alloc(w.nf, st));
-    k_ingest_emit_records<<<(w.nf + 255) / 256, 256, 0, st>>>(w.v.p, w.faces.p, 0, w.nf, w.fn_unit.p, w.vn.p, w.uv.p,
-                                                             w.nuv, w.ranges.p, w.nm, dt.p, da.p);
-    AZ_CUDA_TRY(cudaGetLastError());
+    if (vertex_normals && w.nv)
+        AZ_CUDA_TRY(cudaMemcpyAsync(vertex_normals, w.vn.p, (size_t)w.nv * 12, cudaMemcpyDeviceToHost, st));
+    if ((tris || attrs) && w.nf) {
+        if (tris) AZ_CUDA_TRY(dt.alloc(w.nf, st));
+        if (attrs) AZ_CUDA_TRY(da.alloc(w.nf, st));
+        k_ingest_emit_records<<<(w.nf + 255) / 256, 256, 0, st>>>(w.v.p, w.faces.p, 0, w.nf, w.fn_unit.p, w.vn.p,
+                                                                 w.uv.p, w.nuv, w.ranges.p, w.nm, dt.p, da.p);
+        AZ_CUDA_TRY(cudaGetLastError());
+        if (tris)
+            AZ_CUDA_TRY(cudaMemcpyAsync(tris, dt.p, (size_t)w.nf * sizeof(az_triangle), cudaMemcpyDeviceToHost, st));
+        if (attrs)
+            AZ_CUDA_TRY(cudaMemcpyAsync(attrs, da.p, (size_t)w.nf * sizeof(az_face_attr), cudaMemcpyDeviceToHost, st));
+    }
     AZ_CUDA_TRY(cudaStreamSynchronize(st));
-    if (tris) AZ_CUDA_TRY(cudaMemcpy(tris, dt.p, (size_t)w.nf * sizeof(az_triangle), cudaMemcpyDeviceToHost));
-    if (attrs) AZ_CUDA_TRY(cudaMemcpy(attrs, da.p, (size_t)w.nf * sizeof(az_face_attr), cudaMemcpyDeviceToHost));
     return AZ_OK;
 }
 
