@@ -345,10 +345,10 @@ extern "C" int az_gpu_render_guided(az_gpu_scene *scene, az_guide *guide, az_pix
     if (!scene || !scene->impl || !guide || !film || !camera) return SetError(AZ_ERR_INVALID_ARGUMENT, "null argument");
     GuideState *g = GuideOf(guide);
     if (!g) return SetError(AZ_ERR_INVALID_ARGUMENT, "null guide");
+    std::lock_guard<std::mutex> lock(GuideLock(*g));   // released after ctx has waited for its stream
     CallContext ctx;
     int rc = ctx.begin(opts);
     if (rc != AZ_OK) return rc;
-    std::lock_guard<std::mutex> lock(GuideLock(*g));
     rc = Render(*scene->impl, film, camera, epsilons, scissor, filter_type, backface_culling, opts, ctx.stream, stats,
                 g, train != 0);
     if (rc == AZ_OK) rc = GuideCheck(*g, ctx.stream);

@@ -1865,6 +1865,7 @@ extern "C" int az_guide_get_params(az_guide *g, float *mlp, float *bias, float *
     if (!g) return SetError(AZ_ERR_INVALID_ARGUMENT, "null guide");
     GuideState &s = *g->impl;
     AZ_CUDA_TRY(cudaSetDevice(s.device));
+    std::lock_guard<std::mutex> lock(s.mu);
     AZ_CUDA_TRY(cudaDeviceSynchronize());
     if (mlp) AZ_CUDA_TRY(cudaMemcpy(mlp, s.w, NW * sizeof(float), cudaMemcpyDeviceToHost));
     if (bias) AZ_CUDA_TRY(cudaMemcpy(bias, s.bias, W * sizeof(float), cudaMemcpyDeviceToHost));
@@ -1876,6 +1877,7 @@ extern "C" int az_guide_set_params(az_guide *g, const float *mlp, const float *b
     if (!g) return SetError(AZ_ERR_INVALID_ARGUMENT, "null guide");
     GuideState &s = *g->impl;
     AZ_CUDA_TRY(cudaSetDevice(s.device));
+    std::lock_guard<std::mutex> lock(s.mu);
     AZ_CUDA_TRY(cudaDeviceSynchronize());
     if (mlp) AZ_CUDA_TRY(cudaMemcpy(s.w, mlp, NW * sizeof(float), cudaMemcpyHostToDevice));
     if (bias) AZ_CUDA_TRY(cudaMemcpy(s.bias, bias, W * sizeof(float), cudaMemcpyHostToDevice));
@@ -1906,6 +1908,7 @@ extern "C" int az_guide_eval(az_guide *g, const float *rows, uint32_t n, float *
     if (!g || (n && !rows)) return SetError(AZ_ERR_INVALID_ARGUMENT, "null argument");
     GuideState &s = *g->impl;
     AZ_CUDA_TRY(cudaSetDevice(s.device));
+    std::lock_guard<std::mutex> lock(s.mu);
     GuideRow *d_rows = nullptr;
     uint32_t *d_count = nullptr;
     float *d_out = nullptr, *d_enc = nullptr;
@@ -1967,6 +1970,7 @@ extern "C" int az_guide_train(az_guide *g, const float *rows, uint32_t n, uint32
     if (!g || (n && !rows)) return SetError(AZ_ERR_INVALID_ARGUMENT, "null argument");
     GuideState &s = *g->impl;
     AZ_CUDA_TRY(cudaSetDevice(s.device));
+    std::lock_guard<std::mutex> lock(s.mu);
     // a blocking stream: after earlier work on the legacy default stream
     cudaStream_t st = nullptr;
     AZ_CUDA_TRY(AcquireStream(&st));
@@ -1979,6 +1983,7 @@ extern "C" int az_guide_infer(az_guide *g, const float *rows, uint32_t n, float 
     if (!g || (n && (!rows || !outputs))) return SetError(AZ_ERR_INVALID_ARGUMENT, "null argument");
     GuideState &s = *g->impl;
     AZ_CUDA_TRY(cudaSetDevice(s.device));
+    std::lock_guard<std::mutex> lock(s.mu);
     if (n == 0) return AZ_OK;
     GuideRow *d_rows = nullptr;
     uint32_t *d_count = nullptr;

@@ -135,7 +135,9 @@ int GuideTrainWave(GuideState &g, const WaveQueues &Q, cudaStream_t st);
 GuideState *GuideOf(az_guide *g);
 // AZ_ERR_CUDA if a tensor-core wait of the proposal kernel gave up since the last check (the flag is cleared).
 int GuideCheck(GuideState &g, cudaStream_t st);
-// Serialises the renders that use one guide (its proposal and record buffers).
+// Serialises the calls that use one guide: renders (its proposal and record buffers),
+// training, evaluation and parameter access, each on a stream of its own.  Held until
+// the call has waited for its stream.
 std::mutex &GuideLock(GuideState &g);
 
 // `guide` (may be null) steers the scattering direction; `train` also

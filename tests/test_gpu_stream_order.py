@@ -1,5 +1,8 @@
-"""Calls on a caller's stream that the legacy default stream does not order (a torch side stream is non-blocking)."""
+"""Calls that no common stream orders: on a caller's non-blocking stream (a torch side stream is one), and of several
+threads, each on a stream of its own."""
 import ctypes as C
+import threading
+import time
 
 import numpy as np
 import pytest
@@ -31,3 +34,38 @@ def test_mesh_postprocess_is_finished_when_it_returns(gpu, want):
     finally:
         for s in scenes:
             s.close()
+
+
+@pytest.mark.parametrize("call", ["train", "infer", "eval", "params"])
+def test_calls_on_one_guide_take_turns(gpu, call):
+    """A call on a guide that another thread renders with begins when that render has ended: it returns later, and
+    the render's film is that of the network before the call (the order of float sums apart: 1e-4)."""
+    import torch
+    scene = az.generate_scene(az.SCENE_INTERIOR, seed=1, width=640, height=360, spp=64, detail=8, max_depth=6)
+    rng = np.random.default_rng(3)
+    rows = np.zeros((4099, 16), np.float32)
+    rows[:, 0:3] = rng.uniform(0.5, 3.5, (4099, 3))
+    rows[:, 3] = 1.0
+    rows[:, 5] = rows[:, 9] = rows[:, 13] = 1.0
+    films = [torch.zeros((360, 640, 4), device="cuda") for _ in range(2)]
+    torch.cuda.synchronize()
+    with az.GpuScene(scene) as g, az.Guide(g, seed=4) as guide:
+        t0 = time.perf_counter()
+        guide.render(films[0].data_ptr(), seed=7)
+        alone = time.perf_counter() - t0
+        end = []
+        thread = threading.Thread(target=lambda: (guide.render(films[1].data_ptr(), seed=7),
+                                                  end.append(time.perf_counter())))
+        thread.start()
+        time.sleep(min(0.02, 0.3 * alone))
+        {"train": lambda: guide.train(rows, 8), "infer": lambda: guide.infer(rows), "eval": lambda: guide.eval(rows),
+         "params": lambda: guide.set_params(*[0.5 * p for p in guide.params()])}[call]()
+        done = time.perf_counter()
+        thread.join()
+    a, b = (f.cpu().numpy() for f in films)
+    floor = 1e-3 * float(np.abs(a[..., :3]).mean())
+    err = (np.abs(a - b) / np.maximum(np.abs(a), floor)).max(axis=-1)
+    print("%s: render %.0f ms, the call ended %.1f ms after it" % (call, 1e3 * alone, 1e3 * (done - end[0])))
+    assert alone > 0.04 and done > end[0] - 1e-3
+    assert (err <= 1e-4).mean() >= 0.999
+    scene.close()
