@@ -905,8 +905,9 @@ static int ReplayWave(const GpuScene &G, const CameraParams &cam, WaveBuffers &W
     return AZ_OK;
 }
 
+// in kVariants: {0, 32}, {8, 32}, {8, 8}, {8, 12}
+constexpr uint32_t kLoop = 10, kTogether = 9, kEight = 7, kTwelve = 3;
 void ChooseDefaultVariants(GpuScene &G) {
-    constexpr uint32_t kLoop = 10, kTogether = 9, kEight = 7, kTwelve = 3;   // {0, 32}, {8, 32}, {8, 8}, {8, 12}
     // Scenes of a few nodes (Cornell box 1 + 1, 1 M samples: 1.61 ms a frame
     // with one query per thread, 1.82 by phases).  The visibility queries of
     // several kinds of light take different paths in a warp all the same (the
@@ -925,11 +926,16 @@ void ChooseDefaultVariants(GpuScene &G) {
 }
 
 // The launch configurations of a render: the one the caller names (for both
-// traversal kernels), else the scene's.
-static int ChooseVariants(const GpuScene &G, const az_render_opts *opts, CameraParams &cam) {
+// traversal kernels), else the scene's.  A wave of several scenes has no form
+// with one query per thread, so it takes the default lanes for a scene's that
+// is meant for it: with all 32 lanes waiting for each other, 24 jobs of three
+// scenes take 25.6 ms, with 8 and 12 18.8.
+static int ChooseVariants(const GpuScene &G, const az_render_opts *opts, CameraParams &cam, bool several = false) {
     cam.variant = opts && opts->variant ? opts->variant - 1 : G.variant;
     if (cam.variant >= kVariantCount) return SetError(AZ_ERR_INVALID_ARGUMENT, "unknown launch variant");
     cam.shadow_variant = (opts && opts->variant) || G.shadow_variant >= kVariantCount ? cam.variant : G.shadow_variant;
+    if (several && kVariants[cam.variant].minb == 0) cam.variant = kEight;
+    if (several && kVariants[cam.shadow_variant].minb == 0) cam.shadow_variant = kTwelve;
     cam.refill = kVariants[cam.variant].refill;
     cam.shadow_refill = kVariants[cam.shadow_variant].refill;
     return AZ_OK;
@@ -1113,11 +1119,14 @@ int RenderTiles(GpuScene &G, std::vector<TileJob> &jobs, const az_render_opts *o
     }
     const bool multi = scenes.size() > 1;
     // the record the launches are chosen for: the first scene's, with the
-    // features, light kinds and depth of all of them
+    // features, light kinds and depth of all of them; the launch configuration
+    // is that of the scene with the most nodes, whose queries take the time
     DevScene wave_dev = scenes[0]->dev;
+    const GpuScene *largest = scenes[0];
     uint32_t per_node_shadow = 0;
     for (GpuScene *sg : scenes) {
         const DevScene &d = sg->dev;
+        if (sg->node_count > largest->node_count) largest = sg;
         if (d.max_depth + 1 > AZ_MAX_LEVELS - 2) return SetError(AZ_ERR_UNSUPPORTED, "MaxRecursionDepth above 61");
         wave_dev.features |= d.features;
         wave_dev.full_light_queries |= d.full_light_queries;
@@ -1138,7 +1147,7 @@ int RenderTiles(GpuScene &G, std::vector<TileJob> &jobs, const az_render_opts *o
         c.scene = scene_of[j];
         c.count_traversal = opts && (opts->flags & AZ_FLAG_COUNT_TRAVERSAL) ? 1u : 0u;
         c.env_importance = opts && (opts->flags & AZ_FLAG_ENV_IMPORTANCE) && Gj.dev.env_rows ? 1u : 0u;
-        if ((rc = ChooseVariants(G, opts, c)) != AZ_OK) return rc;
+        if ((rc = ChooseVariants(*largest, opts, c, multi)) != AZ_OK) return rc;
         // several scenes: no queue ordering (its keys use one scene's bounds)
         c.order = multi ? 0u : QueueOrder(G, opts);
         c.serial_levels = opts && (opts->flags & AZ_FLAG_SERIAL_LEVELS) ? 1u : 0u;
