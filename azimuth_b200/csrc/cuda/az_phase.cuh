@@ -41,16 +41,6 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
     return r;
 }
 
-// safe_inv with the hardware's approximate reciprocal (1 ulp): the box tests
-// have half a grid step of slack.
-__device__ __forceinline__ float rcp_box(float x) {
-    const float tiny = 1e-18f;
-    float r;
-    x = fabsf(x) < tiny ? copysignf(tiny, x) : x;
-    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-
 struct WideHits2 {
     uint32_t inner;      // hit inner children, bit = slot ^ perm
     uint32_t lo, hi;     // meta bytes of the hit leaf children, slots 0-3 and 4-7
@@ -164,7 +154,7 @@ struct PhaseTracer {
         o = r.o;
         d = r.d;
         if (SPH) time = r.time;
-        inv = mk(rcp_box(d.x), rcp_box(d.y), rcp_box(d.z));
+        inv = safe_inv(d);
         perm = octant_of(d) ^ (KIND == Q_ANY ? 0u : 7u);
         if (WT) wt = wt_setup(d);
     }

@@ -32,7 +32,8 @@ def _entity(addr):
 
 
 def _scale_instances(scene, factors):
-    """Gives the scene's k-th mesh instance the scale factors[k % len(factors)] and refits the tree's boxes."""
+    """Gives the scene's k-th mesh instance the scale factors[k % len(factors)], one for all axes or one each, and
+    refits the tree's boxes."""
     turn = [0]
 
     def visit(e):
@@ -47,8 +48,8 @@ def _scale_instances(scene, factors):
             s = factors[turn[0] % len(factors)]
             turn[0] += 1
             _floats(e + TRANSFORM, 16)[[0, 5, 10]] = s
-            _floats(e + INVERSE, 16)[[0, 5, 10]] = 1.0 / s
-            box[:] *= s
+            _floats(e + INVERSE, 16)[[0, 5, 10]] = 1.0 / np.asarray(s)
+            box.reshape(3, 3)[:] *= s
         return box
 
     visit(C.c_void_p.from_address(scene.scene_ptr + BVH_ROOT).value)
@@ -56,12 +57,13 @@ def _scale_instances(scene, factors):
 
 def _set_lights(scene, scale):
     """A point, an area and a spot light instead of the scene's own; returns what holds them."""
+    s = np.ones(3) * scale
     buf = (C.c_ubyte * (3 * LIGHT_SIZE))()
     base = C.addressof(buf)
-    _floats(base, 6)[:] = [4 * scale, 3.4 * scale, 2 * scale, 90, 80, 70]                       # point, room 1
-    _floats(base + LIGHT_SIZE, 15)[:] = [20 * scale, 3.7 * scale, 5 * scale, 60, 65, 70,        # area, room 3
-                                         scale, 0, 0, 0, 0, scale, 0, -1, 0]
-    _floats(base + 2 * LIGHT_SIZE, 13)[:] = [12.4 * scale, 3.8 * scale, 0.5 * scale, 200, 190, 150,   # spot, room 2
+    _floats(base, 6)[:] = [*(s * [4, 3.4, 2]), 90, 80, 70]                                      # point, room 1
+    _floats(base + LIGHT_SIZE, 15)[:] = [*(s * [20, 3.7, 5]), 60, 65, 70,                       # area, room 3
+                                         s[0], 0, 0, 0, 0, s[2], 0, -1, 0]
+    _floats(base + 2 * LIGHT_SIZE, 13)[:] = [*(s * [12.4, 3.8, 0.5]), 200, 190, 150,            # spot, room 2
                                              0.3, -0.5, 1, 80, 60, np.cos(np.radians(40)), np.cos(np.radians(30))]
     for k, kind in enumerate((0, 1, 3)):
         C.c_uint32.from_address(base + k * LIGHT_SIZE + LIGHT_TYPE).value = kind
@@ -73,6 +75,24 @@ def _set_lights(scene, scale):
 FACTORS = {"identity": [1.0], "doubled": [2.0], "halved": [0.5], "by turns": [1.0, 2.0]}
 
 
+def _lit_interior(scale, seed=3):
+    """The interior under the three lights, its instances scaled; and a function that puts the scene back."""
+    scene = az.generate_scene(az.SCENE_INTERIOR, seed=seed, width=96, height=54, spp=4, max_depth=2, detail=4)
+    own = (C.c_void_p.from_address(scene.scene_ptr + LIGHTS).value,
+           C.c_uint32.from_address(scene.scene_ptr + LIGHT_COUNT).value)
+    _scale_instances(scene, [scale])
+    lights = _set_lights(scene, scale)
+    _floats(scene.camera_ptr + CAMERA_POSITION, 3)[:] *= scale
+
+    def close():
+        nonlocal lights
+        C.c_void_p.from_address(scene.scene_ptr + LIGHTS).value, lights = own[0], None
+        C.c_uint32.from_address(scene.scene_ptr + LIGHT_COUNT).value = own[1]
+        scene.close()
+
+    return scene, close
+
+
 @pytest.mark.parametrize("flags", [0, az.FLAG_WATERTIGHT], ids=["cramer", "watertight"])
 @pytest.mark.parametrize("case,variant", [("identity", 0), ("identity", 11), ("doubled", 0), ("doubled", 11),
                                           ("halved", 0)])   # 11: one query per thread
@@ -80,14 +100,8 @@ def test_shadows_of_lights_many_units_away(gpu, case, variant, flags):
     """The film's bar is that of the parity tests (1e-4 on all but a few pixels); the watertight test may also take
     the other side of a shared edge.  An occluder that is missed changes a pixel by the whole of a light."""
     import torch
-    s = FACTORS[case][0]
-    scene = az.generate_scene(az.SCENE_INTERIOR, seed=3, width=96, height=54, spp=4, max_depth=2, detail=4)
-    keep = (scene.scene_ptr, LIGHTS, C.c_void_p.from_address(scene.scene_ptr + LIGHTS).value,
-            C.c_uint32.from_address(scene.scene_ptr + LIGHT_COUNT).value)
+    scene, close = _lit_interior(FACTORS[case][0])
     try:
-        _scale_instances(scene, FACTORS[case])
-        lights = _set_lights(scene, s)
-        _floats(scene.camera_ptr + CAMERA_POSITION, 3)[:] *= s
         want = ol.port_film(scene, seed=5)
         film = torch.zeros((54, 96, 4), device="cuda")
         with az.GpuScene(scene) as g:
@@ -95,11 +109,33 @@ def test_shadows_of_lights_many_units_away(gpu, case, variant, flags):
         ok, _, relmse = ol.film_compare(film.cpu().numpy(), want, 1e-4)
         print("%s: pixels within 1e-4 %.4f, relMSE %.3e" % (case, ok, relmse))
         assert ok >= (0.97 if flags else 0.99)
-        del lights
     finally:
-        C.c_void_p.from_address(keep[0] + keep[1]).value = keep[2]
-        C.c_uint32.from_address(keep[0] + LIGHT_COUNT).value = keep[3]
-        scene.close()
+        close()
+
+
+@pytest.mark.parametrize("scale", [(40.0, 1.0, 0.05), (0.02, 30.0, 1.0)], ids=["long", "tall"])
+def test_long_thin_boxes_and_distant_origins(gpu, scale):
+    """Node boxes a thousand times as long as wide, and origins far from them in units of their width: the box tests'
+    rounding stays inside the boxes' slack.  The phases find what one query per thread finds (1e-5 of the largest
+    sum), and both what the restatement finds, with the parity tests' bar."""
+    import torch
+    scene, close = _lit_interior(np.array(scale))
+    try:
+        want = ol.port_film(scene, seed=6)
+        assert (want[..., :3].max(axis=-1) > 0.0).mean() > 0.5
+        films = []
+        with az.GpuScene(scene) as g:
+            for variant in (11, 0, 8, 20):
+                film = torch.zeros((54, 96, 4), device="cuda")
+                g.render_device(film.data_ptr(), seed=6, variant=variant)
+                films.append(film.cpu().numpy())
+        for f in films[1:]:
+            assert np.abs(f - films[0]).max() <= 1e-5 * np.abs(films[0]).max()
+        ok, _, relmse = ol.film_compare(films[1], want, 1e-4)
+        print("%s: pixels within 1e-4 %.4f, relMSE %.3e" % (scale, ok, relmse))
+        assert ok >= 0.99
+    finally:
+        close()
 
 
 @pytest.mark.parametrize("length", [0.1, 1.0, 10.0])
