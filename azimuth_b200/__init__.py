@@ -553,3 +553,8 @@ def device_info(device=0):
     buf = C.create_string_buffer(256)
     rc = lib().az_gpu_device_info(device, buf, 256)
     return buf.value.decode() if rc == 0 else None
+
+
+def release_memory(device=0):
+    """az_gpu_release_memory: gives back the memory and streams that the library keeps between calls."""
+    _check(lib().az_gpu_release_memory(device), "az_gpu_release_memory")

@@ -210,6 +210,8 @@ def _declare(L):
         L.az_gpu_closest_hit.restype = i32
         L.az_gpu_device_info.argtypes = [i32, vp, u32]
         L.az_gpu_device_info.restype = i32
+        L.az_gpu_release_memory.argtypes = [i32]
+        L.az_gpu_release_memory.restype = i32
         L.az_rng_u01.argtypes = [u64, u32, u32, u32, u32, u32]
         L.az_rng_u01.restype = C.c_float
         L.az_rng_philox4x32_10.argtypes = [vp, u32, u32, vp]

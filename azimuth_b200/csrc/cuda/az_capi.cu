@@ -83,6 +83,18 @@ extern "C" int az_gpu_device_info(int32_t device, char *name, uint32_t name_len)
     return AZ_OK;
 }
 
+extern "C" int az_gpu_release_memory(int32_t device) {
+    int n = 0;
+    if (cudaGetDeviceCount(&n) != cudaSuccess || n == 0) {
+        cudaGetLastError();
+        return SetError(AZ_ERR_NO_DEVICE, "no CUDA device available");
+    }
+    if (device < 0 || device >= n) return SetError(AZ_ERR_INVALID_ARGUMENT, "device ordinal out of range");
+    AZ_CUDA_TRY(cudaSetDevice(device));
+    AZ_CUDA_TRY(PoolRelease());
+    return AZ_OK;
+}
+
 extern "C" int az_gpu_scene_create(const az_scene *scene, const az_render_opts *opts, az_gpu_scene **out) {
     if (!scene || !out) return SetError(AZ_ERR_INVALID_ARGUMENT, "null argument");
     *out = nullptr;

@@ -1427,7 +1427,7 @@ struct GuideState {
     template <typename T>
     T *Alloc(size_t n) {
         void *p = nullptr;
-        if (cudaMalloc(&p, n * sizeof(T)) != cudaSuccess) return nullptr;
+        if (DeviceAlloc(&p, n * sizeof(T)) != cudaSuccess) return nullptr;
         allocs.push_back(p);
         return (T *)p;
     }
@@ -1743,8 +1743,8 @@ static int OrderRows(GuideState &g, const WaveQueues &Q, uint32_t level, cudaStr
             *p = nullptr;
         }
         g.row_cap = 0;
-        if (cudaMalloc((void **)&g.row_keys, (size_t)Q.cap_q * sizeof(uint32_t)) != cudaSuccess ||
-            cudaMalloc((void **)&g.row_order, (size_t)Q.cap_q * sizeof(uint32_t)) != cudaSuccess)
+        if (DeviceAlloc((void **)&g.row_keys, (size_t)Q.cap_q * sizeof(uint32_t)) != cudaSuccess ||
+            DeviceAlloc((void **)&g.row_order, (size_t)Q.cap_q * sizeof(uint32_t)) != cudaSuccess)
             return SetError(AZ_ERR_OUT_OF_MEMORY, "path guide row order");
         g.row_cap = Q.cap_q;
     }
@@ -1784,11 +1784,11 @@ int GuideTrainWave(GuideState &g, const WaveQueues &Q, cudaStream_t st) {
         AZ_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, g.rec_flag, g.rec_pos, (int)total));
         AZ_CUDA_TRY(cub::DeviceReduce::Sum(nullptr, sum_bytes, g.kept_weight, g.wsum, (int)g.rows_cap));
         g.cub_bytes = std::max(scan_bytes, sum_bytes);
-        if (cudaMalloc((void **)&g.rec_weight, (size_t)total * sizeof(float) + (size_t)g.rows_cap * sizeof(float)) !=
+        if (DeviceAlloc((void **)&g.rec_weight, (size_t)total * sizeof(float) + (size_t)g.rows_cap * sizeof(float)) !=
                 cudaSuccess ||
-            cudaMalloc((void **)&g.rec_flag, (size_t)total * sizeof(uint32_t)) != cudaSuccess ||
-            cudaMalloc((void **)&g.rec_pos, (size_t)total * sizeof(uint32_t)) != cudaSuccess ||
-            cudaMalloc(&g.cub_temp, g.cub_bytes) != cudaSuccess)
+            DeviceAlloc((void **)&g.rec_flag, (size_t)total * sizeof(uint32_t)) != cudaSuccess ||
+            DeviceAlloc((void **)&g.rec_pos, (size_t)total * sizeof(uint32_t)) != cudaSuccess ||
+            DeviceAlloc(&g.cub_temp, g.cub_bytes) != cudaSuccess)
             return SetError(AZ_ERR_OUT_OF_MEMORY, "path guide training scratch");
         g.rec_cap = total;
     }
@@ -1896,8 +1896,8 @@ extern "C" int az_guide_set_params(az_guide *g, const float *mlp, const float *b
 static int UploadRows(GuideState &s, const float *rows, uint32_t n, GuideRow **d_rows, uint32_t **d_count) {
     *d_rows = nullptr;
     *d_count = nullptr;
-    AZ_CUDA_TRY(cudaMalloc((void **)d_rows, std::max<size_t>(n, 1) * sizeof(GuideRow)));
-    AZ_CUDA_TRY(cudaMalloc((void **)d_count, sizeof(uint32_t)));
+    AZ_CUDA_TRY(DeviceAlloc((void **)d_rows, std::max<size_t>(n, 1) * sizeof(GuideRow)));
+    AZ_CUDA_TRY(DeviceAlloc((void **)d_count, sizeof(uint32_t)));
     AZ_CUDA_TRY(cudaMemcpy(*d_rows, rows, (size_t)n * sizeof(GuideRow), cudaMemcpyHostToDevice));
     AZ_CUDA_TRY(cudaMemcpy(*d_count, &n, sizeof(uint32_t), cudaMemcpyHostToDevice));
     return AZ_OK;
@@ -1913,9 +1913,9 @@ extern "C" int az_guide_eval(az_guide *g, const float *rows, uint32_t n, float *
     uint32_t *d_count = nullptr;
     float *d_out = nullptr, *d_enc = nullptr;
     int rc = UploadRows(s, rows, n, &d_rows, &d_count);
-    if (rc == AZ_OK && outputs && cudaMalloc((void **)&d_out, std::max<size_t>(n, 1) * W * sizeof(float)) != cudaSuccess)
+    if (rc == AZ_OK && outputs && DeviceAlloc((void **)&d_out, std::max<size_t>(n, 1) * W * sizeof(float)) != cudaSuccess)
         rc = SetError(AZ_ERR_OUT_OF_MEMORY, "eval outputs");
-    if (rc == AZ_OK && enc_grad && cudaMalloc((void **)&d_enc, std::max<size_t>(n, 1) * 32 * sizeof(float)) != cudaSuccess)
+    if (rc == AZ_OK && enc_grad && DeviceAlloc((void **)&d_enc, std::max<size_t>(n, 1) * 32 * sizeof(float)) != cudaSuccess)
         rc = SetError(AZ_ERR_OUT_OF_MEMORY, "eval gradients");
     if (rc == AZ_OK) {
         cudaMemset(s.w_grad, 0, NW * sizeof(float));
@@ -1989,7 +1989,7 @@ extern "C" int az_guide_infer(az_guide *g, const float *rows, uint32_t n, float 
     uint32_t *d_count = nullptr;
     float *d_out = nullptr;
     int rc = UploadRows(s, rows, n, &d_rows, &d_count);
-    if (rc == AZ_OK && cudaMalloc((void **)&d_out, (size_t)n * W * sizeof(float)) != cudaSuccess)
+    if (rc == AZ_OK && DeviceAlloc((void **)&d_out, (size_t)n * W * sizeof(float)) != cudaSuccess)
         rc = SetError(AZ_ERR_OUT_OF_MEMORY, "inference outputs");
     if (rc == AZ_OK) {
         cudaMemset(s.tc_error, 0, sizeof(uint32_t));

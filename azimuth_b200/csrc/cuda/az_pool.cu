@@ -50,26 +50,56 @@ cudaError_t PoolOf(int dev, cudaMemPool_t *out) {
 
 }  // namespace
 
+// What the pool keeps may be in the way of an allocation: gives it back once the
+// frees queued on `st` and without a stream have finished.
+static void Trim(int dev, cudaStream_t st) {
+    cudaGetLastError();
+    cudaStream_t idle = nullptr;
+    cudaMemPool_t pool = nullptr;
+    {
+        DevicePools &P = Pools();
+        std::lock_guard<std::mutex> lock(P.mu);
+        if (dev < 0 || dev >= kMaxDevices || !P.pool[dev]) return;
+        pool = P.pool[dev];
+        idle = P.idle[dev];
+    }
+    if (idle) cudaStreamSynchronize(idle);
+    if (st) cudaStreamSynchronize(st);
+    cudaMemPoolTrimTo(pool, 0);
+    cudaGetLastError();
+}
+
+static cudaError_t AllocTrimmed(void **p, size_t bytes, int dev, cudaStream_t st) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        Trim(dev, st);
+        e = cudaMalloc(p, bytes);
+    }
+    if (e != cudaSuccess) {
+        *p = nullptr;
+        cudaGetLastError();
+    }
+    return e;
+}
+
+cudaError_t DeviceAlloc(void **p, size_t bytes) {
+    *p = nullptr;
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    return e == cudaSuccess ? AllocTrimmed(p, bytes, dev, nullptr) : e;
+}
+
 cudaError_t PoolAlloc(void **p, size_t bytes, cudaStream_t st) {
     *p = nullptr;
     int dev = 0;
     cudaMemPool_t pool = nullptr;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess && bytes > kPoolLargest) {
-        e = cudaMalloc(p, bytes);
-        if (e == cudaErrorMemoryAllocation) {
-            // what the pool keeps may be in the way
-            cudaGetLastError();
-            if (PoolOf(dev, &pool) == cudaSuccess && cudaStreamSynchronize(st) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
-            e = cudaMalloc(p, bytes);
-        }
+        e = AllocTrimmed(p, bytes, dev, st);
         if (e == cudaSuccess) {
             DevicePools &P = Pools();
             std::lock_guard<std::mutex> lock(P.mu);
             P.direct.insert(*p);
-        } else {
-            *p = nullptr;
-            cudaGetLastError();
         }
         return e;
     }
@@ -77,10 +107,7 @@ cudaError_t PoolAlloc(void **p, size_t bytes, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     e = cudaMallocFromPoolAsync(p, bytes, pool, st);
     if (e == cudaErrorMemoryAllocation) {
-        // what the pool keeps may be in the way of a large buffer
-        cudaGetLastError();
-        cudaStreamSynchronize(st);
-        cudaMemPoolTrimTo(pool, 0);
+        Trim(dev, st);
         e = cudaMallocFromPoolAsync(p, bytes, pool, st);
     }
     if (e != cudaSuccess) {
@@ -88,6 +115,46 @@ cudaError_t PoolAlloc(void **p, size_t bytes, cudaStream_t st) {
         cudaGetLastError();
     }
     return e;
+}
+
+size_t PoolUnused() {
+    int dev = 0;
+    cudaMemPool_t pool = nullptr;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices) {
+        DevicePools &P = Pools();
+        std::lock_guard<std::mutex> lock(P.mu);
+        pool = P.pool[dev];
+    }
+    unsigned long long reserved = 0, used = 0;
+    if (!pool || cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return reserved > used ? (size_t)(reserved - used) : 0;
+}
+
+cudaError_t PoolRelease() {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    if (e != cudaSuccess || dev < 0 || dev >= kMaxDevices) return e;
+    std::vector<cudaStream_t> streams;
+    std::vector<SideStream> sides;
+    {
+        DevicePools &P = Pools();
+        std::lock_guard<std::mutex> lock(P.mu);
+        streams.swap(P.streams[dev]);
+        sides.swap(P.sides[dev]);
+    }
+    for (cudaStream_t s : streams) cudaStreamDestroy(s);
+    for (const SideStream &s : sides) {
+        cudaEventDestroy(s.fork);
+        cudaEventDestroy(s.join);
+        cudaStreamDestroy(s.stream);
+    }
+    Trim(dev, nullptr);
+    return cudaSuccess;
 }
 
 void PoolFree(void *p, cudaStream_t st) {

@@ -23,6 +23,12 @@ constexpr size_t kPoolKept = (size_t)2 << 30;
 // largest, a build of 1.3 M triangles: 62 MB).
 constexpr size_t kPoolLargest = (size_t)128 << 20;
 cudaError_t PoolAlloc(void **p, size_t bytes, cudaStream_t st);
+// cudaMalloc, tried again after the pool has given back what it keeps unused.
+cudaError_t DeviceAlloc(void **p, size_t bytes);
+// Bytes that the current device's pool keeps unused (cudaMemGetInfo counts them as taken).
+size_t PoolUnused();
+// Waits for the current device and gives back all that is kept on it: the pool's unused memory and the idle streams.
+cudaError_t PoolRelease();
 // Gives memory back once the work queued on `st` so far has finished; no
 // stream: when nothing uses the memory any more.
 void PoolFree(void *p, cudaStream_t st);

@@ -954,8 +954,8 @@ static uint32_t QueueOrder(const GpuScene &G, const az_render_opts *opts) {
 // free device memory holds in wave queues, a power of two from 2^22 to 2^26.
 // Bigger waves keep the launches of the deep tree levels, where most paths
 // have ended, full (C1: 427 ms per frame at 2^22, 393 at 2^24, 383 at 2^26).
-// The queues `W` already holds count as free, so that repeated renders of a
-// scene keep their wave size.
+// The queues `W` already holds and what the pool keeps unused count as free, so
+// that repeated renders of a scene keep their wave size.
 static uint32_t DefaultWave(uint32_t per_node_shadow, const WaveBuffers &W, uint64_t total) {
     uint64_t n = 1u << 22;
     if (total <= n) return (uint32_t)n;   // one wave of the smallest size holds the render
@@ -970,7 +970,7 @@ static uint32_t DefaultWave(uint32_t per_node_shadow, const WaveBuffers &W, uint
     const double per_sample = 1.5 * 168.0 + shadow_entries * 52.0 + 16.0;
     const double held = W.ptrs.empty() ? 0.0
                                        : (double)W.q.cap_q * 168.0 + (double)W.q.cap_s * 52.0 + (double)W.chunk * 16.0;
-    const uint64_t fit = (uint64_t)(((double)free_b + held) / 4.0 / per_sample);
+    const uint64_t fit = (uint64_t)(((double)free_b + (double)PoolUnused() + held) / 4.0 / per_sample);
     while (n * 2 <= fit && n < (1u << 26)) n *= 2;
     return (uint32_t)n;
 }
@@ -1306,7 +1306,7 @@ int Autotune(GpuScene &G, const az_camera *camera, const az_epsilon_values *eps,
     band.Max.x = cam.c0 + cam.wsc;
     size_t bytes = (size_t)cam.width * cam.height * sizeof(az_pixel);
     az_pixel *film = nullptr;
-    AZ_CUDA_TRY(cudaMalloc((void **)&film, bytes));
+    AZ_CUDA_TRY(DeviceAlloc((void **)&film, bytes));
     float best_ms = FLT_MAX;
     uint32_t best = 0;
     az_render_opts o;

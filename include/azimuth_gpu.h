@@ -476,6 +476,13 @@ int az_gpu_closest_hit(az_gpu_scene *scene, const az_ray3 *rays, uint32_t count,
 /* Device name, SM count and memory; returns AZ_ERR_NO_DEVICE without a GPU. */
 int az_gpu_device_info(int32_t device, char *name, uint32_t name_len);
 
+/* Gives back to the driver what the library keeps on a device between calls:
+ * up to 2 GiB of the memory that calls and destroyed scenes gave up, and idle
+ * streams.  Waits for the device; scenes, guides and running calls are not
+ * touched, and the next call takes again what it needs.  For hosts whose other
+ * allocations need that memory (the library's own try again without it). */
+int az_gpu_release_memory(int32_t device);
+
 /* The counter RNG on the host: draw `dim` of tree node (level, digits) of
  * camera sample `sample` (SampleY<<16|SampleX) of pixel `pixel` (Row<<16|Col),
  * exactly as the kernels draw it; and the raw Philox-4x32-10 block function. */
