@@ -23,8 +23,6 @@ constexpr uint32_t AZ_COUNT_SNODES = 2 * AZ_MAX_LEVELS + 5; // visibility querie
 constexpr uint32_t AZ_COUNT_FETCH = 2 * AZ_MAX_LEVELS + 8;  // per level: extend, then shadow work counters
 constexpr uint32_t AZ_COUNT_TOTAL = 4 * AZ_MAX_LEVELS + 8;
 
-// Camera and film parameters of one render call (ProduceImageInLinearSpace's
-// locals, src/azimuth_main.cpp:1265-1347).
 // Division of 32-bit numbers by a number that a launch keeps (Granlund,
 // Montgomery, "Division by Invariant Integers using Multiplication", PLDI
 // 1994): the quotient from a 64-bit product, for every dividend.
@@ -44,6 +42,8 @@ struct FastDiv {
     }
 };
 
+// Camera and film parameters of one render call (ProduceImageInLinearSpace's
+// locals, src/azimuth_main.cpp:1265-1347).
 struct CameraParams {
     azd::f3 base, pos, axx, axy, stepx, stepy;
     float aperture, inv_sqrt;

@@ -238,7 +238,10 @@ enum QueryKind : uint32_t {
 };
 
 // A valid hierarchy needs far fewer steps; the cap only guards against a
-// corrupt one looping forever.  When hit, the query stops and sets *err.
+// corrupt one looping forever.  When hit, the query stops and sets *err.  A
+// thread with a query of its own counts its steps; a warp of the phases counts
+// rounds since it last took queries, so there a query that loops ends once the
+// warp's share of the queue has drained.
 #define AZD_MAX_STEPS (1u << 22)
 #define AZD_WSTACK 48
 
