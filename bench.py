@@ -43,11 +43,11 @@ SCENE_ARGS = dict(scene_id=1, seed=0)
 # one single-pass ncu capture (dram__bytes_read.sum + dram__bytes_write.sum)
 # of every k_extend / k_shadow launch of one 256x256, 16-spp frame (one wave of
 # 2^20 samples): the capture's bytes over the frame's queries
-DRAM_BYTES_PER_QUERY = {"k_extend": 207.1, "k_shadow": 246.2}
+DRAM_BYTES_PER_QUERY = {"k_extend": 187.1, "k_shadow": 186.2}   # k_shadow: with k_light_limits before it
 PROFILE_NOTE = "profiles/traversal_dram_dense_mesh_256x256_16spp.md, profiles/phase_traversal_dense_mesh_256x256_16spp.md"
 # issue statistics of the two traversal kernels from the ncu capture of that small case
-ISSUE = {"k_extend": {"threads_per_warp_instruction": 16.76, "issue_active_pct": 58.3, "warps_active_pct": 41.6},
-         "k_shadow": {"threads_per_warp_instruction": 16.91, "issue_active_pct": 52.3, "warps_active_pct": 41.3}}
+ISSUE = {"k_extend": {"threads_per_warp_instruction": 16.70, "issue_active_pct": 57.2, "warps_active_pct": 41.5},
+         "k_shadow": {"threads_per_warp_instruction": 16.86, "issue_active_pct": 54.0, "warps_active_pct": 41.2}}
 
 
 def parse():
@@ -359,7 +359,7 @@ def main():
     sh_traffic = (DRAM_BYTES_PER_QUERY["k_shadow"] * sh_q / launches_per_frame
                   if dense and DRAM_BYTES_PER_QUERY["k_shadow"] else None)
     limiter = ("instruction issue of divergent traversal, not HBM: about 17 of 32 lanes active per warp "
-               "instruction, DRAM traffic a quarter of the algorithmic bytes (%s)" % PROFILE_NOTE)
+               "instruction, DRAM traffic a fifth of the algorithmic bytes (%s)" % PROFILE_NOTE)
     roofline = {"bound": "hbm", "achieved": ext_achieved, "peak": hbm, "unit": "GB/s", "frac": ext_achieved / hbm,
                 "traffic": ext_traffic, "traffic_unit": "DRAM bytes per launch (ncu, scaled from a small frame)",
                 "algorithmic_bytes_per_launch": ext_bytes / launches_per_frame,
