@@ -18,7 +18,6 @@
 #include <memory>
 #include <set>
 #include <string>
-#include <system_error>
 #include <thread>
 
 #include "az_internal.h"
@@ -292,8 +291,8 @@ struct Flattener {
         for (size_t t = 1; t < want; t++) {
             try {
                 threads.emplace_back(work, t);
-            } catch (const std::system_error &) {
-                break;   // no more threads to be had: the others take the work
+            } catch (...) {
+                break;   // no more threads, or no memory for one: the others take the work
             }
         }
         work(0);
